@@ -15,7 +15,7 @@
 
 namespace rm {
 
-constexpr int kGetriCols = kSolveCols;  // columns of the identity per pair of chain launches
+constexpr int kGetriCols = kSolveCols;  // columns of the identity per chain
 
 __global__ void identity_kernel(double* __restrict__ y, int64_t n) {
   const int64_t total = n * n;
@@ -60,18 +60,11 @@ int getri_f64(const double* f, int64_t n, const int64_t* perm, double* out, void
   const int blocks = (int)std::min<int64_t>((n * n + 255) / 256, 8 * device_sm_count());
   identity_kernel<<<blocks, 256, 0, stream>>>(y, n);
   RM_LAUNCHED();
-  const int ni = (int)n;
-  for (int ch = 0; ch < chunks; ++ch) {
-    const int c0 = ch * kGetriCols, kc = std::min(kGetriCols, ni - c0);
-    // columns c0.. of L^-1 are zero above row c0: the lower solve starts at c0's block row
-    const int b0 = c0 / kSolveBlock, r0 = b0 * kSolveBlock;
-    int* fl = flags + (size_t)ch * 2 * (nblk + 1);
-    RM_TRY(trsv_chain_f64(true, true, f + (int64_t)r0 * n + r0, n, ni - r0,
-                          dinv + (size_t)b0 * kDiagMats * kSolveBlock * kSolveBlock, y + (int64_t)r0 * n + c0, n, kc,
-                          fl, fl + nblk, status, stream));
-    RM_TRY(trsv_chain_f64(false, true, f, n, ni, dinv, y + c0, n, kc, fl + nblk + 1, fl + 2 * nblk + 1, status,
-                          stream));
-  }
+  // chain ch holds columns 16 ch .. of L^-1, zero above row 16 ch: its lower solve starts there
+  const int64_t stride = 2 * (nblk + 1);
+  RM_TRY(trsv_chain_f64(true, true, f, n, (int)n, dinv, y, n, n, flags, flags + nblk, stride, true, status, stream));
+  RM_TRY(trsv_chain_f64(false, true, f, n, (int)n, dinv, y, n, n, flags + nblk + 1, flags + 2 * nblk + 1, stride, false,
+                        status, stream));
   permute_columns_kernel<<<blocks, 256, 0, stream>>>(y, perm, n, out, status);
   RM_LAUNCHED();
   return RM_OK;

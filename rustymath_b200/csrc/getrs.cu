@@ -173,6 +173,14 @@ __device__ __forceinline__ void st_release(int* p, int v) {
 // between seeing p's flag and releasing its own. Thread t owns row t / 4 and columns
 // 4 (t % 4) .. +3 of its block's sums. The next matrix a step needs is loaded into registers
 // while the current one is applied, so each block of T crosses HBM once.
+//
+// A launch runs one chain per kKC columns of x (blockIdx.y), each with its own flags and tickets
+// chain_stride ints apart. A chain is bound by the latency of its handoffs (~5 us a block), not
+// by its products, so the chains of a wide right-hand side run beside each other instead of one
+// launch after another: a CTA only waits for blocks of its own chain whose tickets running CTAs
+// already hold. The inverse of a 1030 x 1030 factorization (65 chains a triangle) took 10.3 ms
+// with a launch per chain. With `identity`, x starts as the identity: chain y's columns are zero
+// above block y * kKC / TB, and the chain starts there (lower triangles only).
 // Shared-memory layout of a chain CTA. float32 with 128-row blocks multiplies on the tensor
 // cores (mma.sync m16n8k8, TF32 inputs split into high and low parts, three products: float32-
 // level accuracy); the padded rows keep its fragment loads free of bank conflicts.
@@ -190,7 +198,8 @@ struct ChainLayout {
 template <typename T, bool LOWER, bool COLMAJOR, int TB, bool PRE>
 __global__ void __launch_bounds__(TB * 4)
     trsv_chain_kernel(const T* __restrict__ w, int64_t ldw, int n, const T* __restrict__ dinv, T* x, int64_t ldx,
-                      int kc, int* flags, int* counter, unsigned* status, uint64_t wait_ns) {
+                      int k, int* flags, int* counter, int64_t chain_stride, bool identity, unsigned* status,
+                      uint64_t wait_ns) {
   using Lay = ChainLayout<T, TB>;
   constexpr int THREADS = TB * 4;
   constexpr int LPT = TB * TB / THREADS;  // items of a block of T per thread
@@ -201,12 +210,18 @@ __global__ void __launch_bounds__(TB * 4)
   __shared__ int ticket;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nblk = (n + TB - 1) / TB;
+  x += (int64_t)blockIdx.y * kKC;
+  flags += (int64_t)blockIdx.y * chain_stride;
+  counter += (int64_t)blockIdx.y * chain_stride;
+  const int kc = min(kKC, k - (int)blockIdx.y * kKC);
+  const int first = LOWER && identity ? (int)blockIdx.y * kKC / TB : 0;  // the chain's first block
   if (tid == 0) ticket = atomicAdd(counter, 1);
   __syncthreads();
   const int t = ticket;
-  const int b = LOWER ? t : nblk - 1 - t;
+  if (t >= nblk - first) return;  // nothing waits on a ticket past the chain's blocks
+  const int b = LOWER ? first + t : nblk - 1 - t;
   const int r0 = b * TB, rows = min(TB, n - r0);
-  auto dep = [&](int s) { return LOWER ? s : nblk - 1 - s; };  // the s-th block solved
+  auto dep = [&](int s) { return LOWER ? first + s : nblk - 1 - s; };  // the s-th block solved
   // this thread's four items of the block's sums: (my_r, my_c + i) for the scalar product; for
   // the tensor-core one, the m16n8 fragment of warp (8 row tiles x 2 column tiles):
   // rows fr + 8 (i >> 1), columns fc + (i & 1)
@@ -384,18 +399,27 @@ __global__ void __launch_bounds__(TB * 4)
   if (tid == 0) st_release(&flags[b], 1);
 }
 
-// Launches one chain (a CTA per block row). `ctas` < 0 launches all of them; the bounded-wait
-// self-test launches one fewer, having taken the first ticket itself.
+// Launches a chain per kKC of x's k columns (a CTA per block row and chain). `ctas` < 0 launches
+// every block row; the bounded-wait self-test launches one fewer, having taken the first ticket
+// itself.
 template <typename T, bool LOWER, bool COLMAJOR, int TB, bool PRE = false>
-static int launch_trsv(const T* w, int64_t ldw, int n, const T* dinv, T* x, int64_t ldx, int kc, int* flags,
-                       int* counter, unsigned* status, cudaStream_t stream, uint64_t wait_ns = kWaitLimitNs,
-                       int ctas = -1) {
+static int launch_trsv(const T* w, int64_t ldw, int n, const T* dinv, T* x, int64_t ldx, int64_t k, int* flags,
+                       int* counter, int64_t chain_stride, unsigned* status, cudaStream_t stream, bool identity = false,
+                       uint64_t wait_ns = kWaitLimitNs, int ctas = -1) {
   const size_t smem = ChainLayout<T, TB>::bytes();
   RM_TRY(smem_attribute(trsv_chain_kernel<T, LOWER, COLMAJOR, TB, PRE>, smem));
   const int nblk = (n + TB - 1) / TB;
-  trsv_chain_kernel<T, LOWER, COLMAJOR, TB, PRE><<<ctas < 0 ? nblk : ctas, TB * 4, smem, stream>>>(
-      w, ldw, n, dinv, x, ldx, kc, flags, counter, status, wait_ns);
-  RM_LAUNCHED();
+  // chains beside each other, as many as a grid's y extent allows
+  constexpr int64_t kMaxChains = 65535;
+  for (int64_t c0 = 0; c0 < k; c0 += kMaxChains * kKC) {
+    const int64_t kc = std::min<int64_t>(k - c0, kMaxChains * kKC), chain0 = c0 / kKC;
+    if (identity && c0 > 0) return RM_BAD_ARG;  // one launch per identity (n < 2^20)
+    const dim3 grid((unsigned)(ctas < 0 ? nblk : ctas), (unsigned)((kc + kKC - 1) / kKC));
+    trsv_chain_kernel<T, LOWER, COLMAJOR, TB, PRE><<<grid, TB * 4, smem, stream>>>(
+        w, ldw, n, dinv, x + c0, ldx, (int)kc, flags + chain0 * chain_stride, counter + chain0 * chain_stride,
+        chain_stride, identity, status, wait_ns);
+    RM_LAUNCHED();
+  }
   return RM_OK;
 }
 
@@ -429,7 +453,7 @@ int chain_timeout_run(uint64_t wait_ns, void* scratch, unsigned* bits, cudaStrea
   RM_TRY((launch_trsv<double, true, false, kTB64>(
       reinterpret_cast<const double*>(base + TimeoutLayout::w), kTimeoutN, kTimeoutN,
       reinterpret_cast<const double*>(base + TimeoutLayout::dinv), reinterpret_cast<double*>(base + TimeoutLayout::x),
-      kKC, kKC, flags, flags + nblk, status, stream, wait_ns, nblk - 1)));
+      kKC, kKC, flags, flags + nblk, nblk + 1, status, stream, false, wait_ns, nblk - 1)));
   RM_CUDA_TRY(cudaMemcpyAsync(bits, status, sizeof(unsigned), cudaMemcpyDeviceToHost, stream));
   RM_CUDA_TRY(cudaStreamSynchronize(stream));
   return RM_OK;
@@ -631,13 +655,19 @@ __global__ void permute_rows_kernel(const double* __restrict__ b, int64_t ldb, c
 }
 
 int trsv_chain_f64(bool lower, bool colmajor, const double* w, int64_t ldw, int n, const double* dinv, double* x,
-                   int64_t ldx, int kc, int* flags, int* counter, unsigned* status, cudaStream_t stream) {
+                   int64_t ldx, int64_t k, int* flags, int* counter, int64_t chain_stride, bool identity,
+                   unsigned* status, cudaStream_t stream) {
   if (lower && colmajor)
-    return launch_trsv<double, true, true, kTB64>(w, ldw, n, dinv, x, ldx, kc, flags, counter, status, stream);
-  if (lower) return launch_trsv<double, true, false, kTB64>(w, ldw, n, dinv, x, ldx, kc, flags, counter, status, stream);
+    return launch_trsv<double, true, true, kTB64>(w, ldw, n, dinv, x, ldx, k, flags, counter, chain_stride, status,
+                                                  stream, identity);
+  if (lower)
+    return launch_trsv<double, true, false, kTB64>(w, ldw, n, dinv, x, ldx, k, flags, counter, chain_stride, status,
+                                                   stream, identity);
   if (colmajor)
-    return launch_trsv<double, false, true, kTB64>(w, ldw, n, dinv, x, ldx, kc, flags, counter, status, stream);
-  return launch_trsv<double, false, false, kTB64>(w, ldw, n, dinv, x, ldx, kc, flags, counter, status, stream);
+    return launch_trsv<double, false, true, kTB64>(w, ldw, n, dinv, x, ldx, k, flags, counter, chain_stride, status,
+                                                   stream);
+  return launch_trsv<double, false, false, kTB64>(w, ldw, n, dinv, x, ldx, k, flags, counter, chain_stride, status,
+                                                  stream);
 }
 
 size_t getrs_f64_scratch_bytes(int64_t n, int64_t k) { return getrs_scratch_bytes_max(n, k); }
@@ -658,21 +688,11 @@ int getrs_f64(const double* lu, int64_t ld, bool lu_colmajor, int64_t n, const i
   const int blocks = (int)std::min<int64_t>((n * k + 255) / 256, 4 * device_sm_count());
   permute_rows_kernel<false><<<blocks, 256, 0, stream>>>(b, ldb, trans ? nullptr : perm, n, k, tmp, k, status);
   RM_LAUNCHED();
-  const int ni = (int)n;
-  for (int ch = 0; ch < chunks; ++ch) {
-    const int kc = (int)std::min<int64_t>(kKC, k - (int64_t)ch * kKC);
-    int* f = flags + (size_t)ch * 2 * (nblk + 1);
-    double* xc = tmp + ch * kKC;
-    if (colmajor) {
-      RM_TRY((launch_trsv<double, true, true, kTB64>(lu, ld, ni, dinv, xc, k, kc, f, f + nblk, status, stream)));
-      RM_TRY((launch_trsv<double, false, true, kTB64>(lu, ld, ni, dinv, xc, k, kc, f + nblk + 1, f + 2 * nblk + 1,
-                                                      status, stream)));
-    } else {
-      RM_TRY((launch_trsv<double, true, false, kTB64>(lu, ld, ni, dinv, xc, k, kc, f, f + nblk, status, stream)));
-      RM_TRY((launch_trsv<double, false, false, kTB64>(lu, ld, ni, dinv, xc, k, kc, f + nblk + 1, f + 2 * nblk + 1,
-                                                       status, stream)));
-    }
-  }
+  const int64_t stride = 2 * (nblk + 1);  // ints per chain: lower flags + ticket, upper flags + ticket
+  RM_TRY(trsv_chain_f64(true, colmajor, lu, ld, (int)n, dinv, tmp, k, k, flags, flags + nblk, stride, false, status,
+                        stream));
+  RM_TRY(trsv_chain_f64(false, colmajor, lu, ld, (int)n, dinv, tmp, k, k, flags + nblk + 1, flags + 2 * nblk + 1, stride,
+                        false, status, stream));
   permute_rows_kernel<true><<<blocks, 256, 0, stream>>>(tmp, k, trans ? perm : nullptr, n, k, x, ldx, status);
   RM_LAUNCHED();
   return RM_OK;
@@ -712,19 +732,8 @@ int trsm_f64(bool right, bool lower, bool trans, bool unit, int64_t m, int64_t n
     y = xt;
     ldy = m;
   }
-  const int no = (int)order;
-  for (int ch = 0; ch < chunks; ++ch) {
-    const int kc = (int)std::min<int64_t>(kKC, cols - (int64_t)ch * kKC);
-    int* f = flags + (size_t)ch * (nblk + 1);
-    double* yc = y + ch * kKC;
-    if (colview) {
-      if (low) RM_TRY((launch_trsv<double, true, true, kTB64>(a, lda, no, dinv, yc, ldy, kc, f, f + nblk, status, stream)));
-      else RM_TRY((launch_trsv<double, false, true, kTB64>(a, lda, no, dinv, yc, ldy, kc, f, f + nblk, status, stream)));
-    } else {
-      if (low) RM_TRY((launch_trsv<double, true, false, kTB64>(a, lda, no, dinv, yc, ldy, kc, f, f + nblk, status, stream)));
-      else RM_TRY((launch_trsv<double, false, false, kTB64>(a, lda, no, dinv, yc, ldy, kc, f, f + nblk, status, stream)));
-    }
-  }
+  RM_TRY(trsv_chain_f64(low, colview, a, lda, (int)order, dinv, y, ldy, cols, flags, flags + nblk, nblk + 1, false,
+                        status, stream));
   if (right) {
     RM_TRY(transpose_f64(xt, m, n, m, x, ldx, stream));
   }
@@ -869,14 +878,10 @@ int lu_solve_f32_nopiv(const float* lu, int64_t ld, int64_t n, const float* dinv
     return launch_trsv_pre_ring<false>(pre, ldp, (int)n, dinv, x, ldx, (int)k, flags + nblk + 1, flags + 2 * nblk + 1,
                                        stride, status, stream);
   }
-  for (int ch = 0; ch < chunks; ++ch) {
-    const int kc = (int)std::min<int64_t>(kKC, k - (int64_t)ch * kKC);
-    int* f = flags + (size_t)ch * stride;
-    float* xc = x + ch * kKC;
-    RM_TRY((launch_trsv<float, true, false, kTB32>(lu, ld, (int)n, dinv, xc, ldx, kc, f, f + nblk, status, stream)));
-    RM_TRY((launch_trsv<float, false, false, kTB32>(lu, ld, (int)n, dinv, xc, ldx, kc, f + nblk + 1, f + 2 * nblk + 1,
-                                                    status, stream)));
-  }
+  RM_TRY((launch_trsv<float, true, false, kTB32>(lu, ld, (int)n, dinv, x, ldx, k, flags, flags + nblk, stride, status,
+                                                 stream)));
+  RM_TRY((launch_trsv<float, false, false, kTB32>(lu, ld, (int)n, dinv, x, ldx, k, flags + nblk + 1,
+                                                  flags + 2 * nblk + 1, stride, status, stream)));
   return RM_OK;
 }
 

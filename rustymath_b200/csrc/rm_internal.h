@@ -103,12 +103,14 @@ int getrs_f64(const double* lu, int64_t ld, bool lu_colmajor, int64_t n, const i
               const double* b, int64_t ldb, int64_t k, double* x, int64_t ldx, void* scratch, unsigned* status,
               cudaStream_t stream, bool trans = false);
 size_t diag_blocks_f64_bytes(int64_t n);
-// One float64 block-chained triangular solve (a CTA per kSolveBlock-row block) of kc <= kSolveCols
-// columns of x in place: the lower or upper triangle of T, T(i, j) at w[i*ldw + j] (w[j*ldw + i]
-// when colmajor), with the diagonal-block inverses of invert_diag_blocks_f64; flags[nblk] and
-// *counter zero on entry.
+// Float64 block-chained triangular solves (a CTA per kSolveBlock-row block) of the k columns of x
+// in place, one chain per kSolveCols of them, side by side: the lower or upper triangle of T,
+// T(i, j) at w[i*ldw + j] (w[j*ldw + i] when colmajor), with the diagonal-block inverses of
+// invert_diag_blocks_f64. Chain c's flags[nblk] and *counter lie c * chain_stride ints on, zero on
+// entry. identity: x is the n x n identity on entry (lower triangles skip its zero blocks).
 int trsv_chain_f64(bool lower, bool colmajor, const double* w, int64_t ldw, int n, const double* dinv, double* x,
-                   int64_t ldx, int kc, int* flags, int* counter, unsigned* status, cudaStream_t stream);
+                   int64_t ldx, int64_t k, int* flags, int* counter, int64_t chain_stride, bool identity,
+                   unsigned* status, cudaStream_t stream);
 // Inverts the diagonal blocks of the lower and upper triangles of T, T(i,j) = w[i*ldw+j]
 // (w[j*ldw+i] when colmajor), a unit triangle's diagonal taken as 1.
 int invert_diag_blocks_f64(const double* w, int64_t ldw, bool colmajor, int64_t n, double* dinv, bool lower_unit,
