@@ -11,6 +11,9 @@
 // thread's register budget to 168 and spill the 64x32 accumulator tile.) The mma row/column each thread's fragment covers
 // is mapped to a tile row/column (fragment maps below) so that every fragment load of a
 // half-warp touches 16 distinct 8-byte bank pairs under the 128-byte swizzle.
+#include <climits>
+
+#include "getrf_block.cuh"
 #include "rm_internal.h"
 
 namespace rm {
@@ -170,21 +173,237 @@ __global__ void __launch_bounds__(C::THREADS, 1)
     return;
   }
 
-  // ---------------- epilogue: C = alpha*acc + beta*C
+  // ---------------- epilogue: C = alpha*acc + beta*C, an m16 row of tiles at a time: all its
+  // items of C are in flight before the first is used
 #pragma unroll
-  for (int i = 0; i < C::MI; ++i)
+  for (int i = 0; i < C::MI; ++i) {
+    double old[C::NJ][4];
+    if (beta != 0.0) {
+#pragma unroll
+      for (int j = 0; j < C::NJ; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int row = m0 + arow(i, g + 8 * (e >> 1)), col = n0 + bcol(j, 2 * t + (e & 1));
+          old[j][e] = row < m && col < n ? c[(int64_t)row * ldc + col] : 0.0;
+        }
+    }
 #pragma unroll
     for (int j = 0; j < C::NJ; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const uint32_t r = g + 8 * (e >> 1), q = 2 * t + (e & 1);
-        const int row = m0 + arow(i, r), col = n0 + bcol(j, q);
-        if (row < m && col < n) {
-          double* p = c + (int64_t)row * ldc + col;
-          const double v = alpha * acc[i][j][e];
-          *p = beta == 0.0 ? v : fma(beta, *p, v);
+        const int row = m0 + arow(i, g + 8 * (e >> 1)), col = n0 + bcol(j, 2 * t + (e & 1));
+        const double v = alpha * acc[i][j][e];
+        if (row < m && col < n) c[(int64_t)row * ldc + col] = beta == 0.0 ? v : fma(beta, old[j][e], v);
+      }
+  }
+}
+
+// ------------------------------------------------------------------ the LU's trailing update
+// C -= A B with A m x k and B k x n row-major and k small (128): a tile's share of C takes nearly a
+// third as long to cross HBM as its products take, so C comes by TMA like the operands, through the
+// tile's products, into a buffer of its own (128 KB; three operand stages beside it). Reading C from
+// global memory at the end, as dgemm_kernel does, ran a 7552 x 7552 rank-128 update at 15.7 TFLOP/s;
+// two CTAs per SM with C read at the start, 23.8; this, 27. The arithmetic is dgemm_kernel's: the
+// products of a tile are summed by themselves and then subtracted from C (starting the sums from C
+// rounds at C's magnitude once per k, and nearly doubled the error of a solve at n = 8192).
+//
+// Persistent: CTAs take tiles from a counter, thread 0 fetching two tiles ahead; it
+// writes a tile into `ring` before it arms the first stage of the tile before it, which every warp
+// waits for, so there is no CTA barrier per tile.
+//
+// A CTA that starts on an SM where the factorization's latest leaf has run (marks) leaves it to the
+// next leaf. While short kernels before it still hold the other SMs, the CTAs yet to start all try
+// those free ones, so the grid is three times the SMs, and all but (SMs - `most`) of its CTAs may
+// leave: the tiles always have that many takers. With one CTA per SM and `most` leaving, the ones
+// turned away came back and kept the marked SMs (n = 8192: 28 ms a factorization against 22).
+using UpdateCfg = DgemmCfg<128, 128, 64, 32, 3, false, false>;
+constexpr int kUpdateC = UpdateCfg::BM * UpdateCfg::BN * 8;
+constexpr size_t kUpdateSmem = UpdateCfg::STAGES * UpdateCfg::STAGE_BYTES + kUpdateC + 1024 + (2 * UpdateCfg::STAGES + 2) * 8;
+
+__global__ void __launch_bounds__(UpdateCfg::THREADS, 1)
+    dgemm_update_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
+                        const __grid_constant__ CUtensorMap tma_c, double* __restrict__ c, int64_t ldc, int m, int n,
+                        int k, const LeafMarks* marks, int may_leave, int* counters, unsigned* status) {
+  using C = UpdateCfg;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* cbuf = smem + C::STAGES * C::STAGE_BYTES;
+  uint64_t* full = reinterpret_cast<uint64_t*>(cbuf + kUpdateC);
+  uint64_t* empty = full + C::STAGES;
+  uint64_t* cfull = empty + C::STAGES;
+  uint64_t* cempty = cfull + 1;
+  __shared__ int ring[4];  // this CTA's tiles, by their order
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ktiles = (k + C::BK - 1) / C::BK;
+  const int tiles_n = (n + C::BN - 1) / C::BN, tiles = tiles_n * ((m + C::BM - 1) / C::BM);
+  griddep_launch_dependents();
+  griddep_wait();  // the kernel before this one in the stream has completed
+  if (threadIdx.x == 0) {
+    unsigned sm;
+    asm("mov.u32 %0, %%smid;" : "=r"(sm));
+    const volatile LeafMarks* mk = marks;
+    const bool leave = sm < kSmMarks && mk->latest != 0 && mk->sm[sm] == mk->latest && atomicAdd(&counters[1], 1) < may_leave;
+    ring[0] = leave ? INT_MAX : atomicAdd(&counters[0], 1);
+    ring[1] = leave ? INT_MAX : atomicAdd(&counters[0], 1);
+    for (int s = 0; s < C::STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], C::COMPUTE_WARPS);
+    }
+    mbar_init(cfull, 1);
+    mbar_init(cempty, C::COMPUTE_WARPS);
+    fence_barrier_init();
+    tma_prefetch_desc(&tma_a);
+    tma_prefetch_desc(&tma_b);
+    tma_prefetch_desc(&tma_c);
+  }
+  __syncthreads();
+  // step st = (tile in this CTA's order) * ktiles + k-tile goes to stage st % STAGES
+  bool producing = true;
+  auto issue = [&](int st, int tile) {
+    const int s = st % C::STAGES;
+    if (st >= C::STAGES && !mbar_wait(&empty[s], ((st - C::STAGES) / C::STAGES) & 1u, status)) {
+      producing = false;
+      return;
+    }
+    uint8_t* sa = smem + s * C::STAGE_BYTES;
+    uint8_t* sb = sa + C::A_BYTES;
+    mbar_arrive_expect_tx(&full[s], C::STAGE_BYTES);
+    const int k0 = st % ktiles * C::BK, m0 = tile / tiles_n * C::BM, n0 = tile % tiles_n * C::BN;
+    tma_load_2d(sa, &tma_a, &full[s], k0, m0);
+#pragma unroll
+    for (int b = 0; b < C::BN / 16; ++b) tma_load_2d(sb + b * 2048, &tma_b, &full[s], n0 + 16 * b, k0);
+  };
+  int c_issued = 0;  // tiles whose C has been asked for
+  auto issue_c = [&](int tile) {
+    if (c_issued > 0 && !mbar_wait(cempty, (c_issued - 1) & 1u, status)) {
+      producing = false;
+      return;
+    }
+    mbar_arrive_expect_tx(cfull, kUpdateC);
+    const int m0 = tile / tiles_n * C::BM, n0 = tile % tiles_n * C::BN;
+#pragma unroll
+    for (int b = 0; b < C::BN / 16; ++b) tma_load_2d(cbuf + b * C::BM * 128, &tma_c, cfull, n0 + 16 * b, m0);
+    ++c_issued;
+  };
+  const int wm0 = (warp / C::WARPS_N) * C::WM, wn0 = (warp % C::WARPS_N) * C::WN;
+  const uint32_t g = lane >> 2, t = lane & 3;
+  auto arow = [&](int i, uint32_t r) -> uint32_t { return wm0 + 16 * i + 2 * (r & 7u) + (r >> 3); };
+  auto bcol = [&](int j, uint32_t q) -> uint32_t { return wn0 + 16 * (j >> 1) + rho(q, j & 1); };
+
+  int tile = ring[0], issued = 0, step = 0;
+  bool ok = true;
+  for (int seq = 0; tile < tiles; ++seq) {
+    int next = ring[(seq + 1) & 3], after = INT_MAX;  // thread 0's own; the others read next below
+    if (threadIdx.x == 0) {
+      after = atomicAdd(&counters[0], 1);
+      for (; issued < step + C::STAGES - 1 && issued < step + ktiles && producing; ++issued) issue(issued, tile);
+      if (producing) issue_c(tile);  // once every warp has read the tile before's
+    }
+    double acc[C::MI][C::NJ][4];
+#pragma unroll
+    for (int i = 0; i < C::MI; ++i)
+#pragma unroll
+      for (int j = 0; j < C::NJ; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.0;
+    const int end = step + ktiles;
+    for (; step < end; ++step) {
+      if (threadIdx.x == 0 && producing) {
+        if (issued < end) {
+          issue(issued, tile), ++issued;
+        } else if (next < tiles && issued < end + ktiles) {
+          if (issued == end) ring[(seq + 2) & 3] = after;
+          issue(issued, next), ++issued;
         }
       }
+      const int s = step % C::STAGES;
+      if (!mbar_wait(&full[s], (step / C::STAGES) & 1u, status)) {
+        ok = false;
+        break;
+      }
+      const uint8_t* sa = smem + s * C::STAGE_BYTES;
+      const uint8_t* sb = sa + C::A_BYTES;
+#pragma unroll
+      for (int kk = 0; kk < C::BK; kk += 8) {
+        double af[C::MI][4], bf[C::NJ][2];
+#pragma unroll
+        for (int i = 0; i < C::MI; ++i) {
+          const uint32_t r0 = arow(i, g), r1 = arow(i, g + 8);
+          af[i][0] = *reinterpret_cast<const double*>(sa + tile_off<true>(r0, kk + t));
+          af[i][1] = *reinterpret_cast<const double*>(sa + tile_off<true>(r1, kk + t));
+          af[i][2] = *reinterpret_cast<const double*>(sa + tile_off<true>(r0, kk + t + 4));
+          af[i][3] = *reinterpret_cast<const double*>(sa + tile_off<true>(r1, kk + t + 4));
+        }
+#pragma unroll
+        for (int j = 0; j < C::NJ; ++j) {
+          const uint32_t q = bcol(j, g);
+          bf[j][0] = *reinterpret_cast<const double*>(sb + tile_off<false>(q, kk + t));
+          bf[j][1] = *reinterpret_cast<const double*>(sb + tile_off<false>(q, kk + t + 4));
+        }
+#pragma unroll
+        for (int i = 0; i < C::MI; ++i)
+#pragma unroll
+          for (int j = 0; j < C::NJ; ++j)
+            asm volatile(
+                "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+                "{%0,%1,%2,%3};"
+                : "+d"(acc[i][j][0]), "+d"(acc[i][j][1]), "+d"(acc[i][j][2]), "+d"(acc[i][j][3])
+                : "d"(af[i][0]), "d"(af[i][1]), "d"(af[i][2]), "d"(af[i][3]), "d"(bf[j][0]), "d"(bf[j][1]));
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[s]);
+    }
+    if (!ok) break;
+    next = ring[(seq + 1) & 3];
+    if (!mbar_wait(cfull, seq & 1u, status)) {
+      ok = false;
+      break;
+    }
+    // rows g and g + 8 of each m16 tile, two neighbouring columns each
+    const int m0 = tile / tiles_n * C::BM, n0 = tile % tiles_n * C::BN;
+#pragma unroll
+    for (int i = 0; i < C::MI; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = arow(i, g + 8 * h), row = m0 + r;
+        double* p = c + (int64_t)row * ldc + n0;
+#pragma unroll
+        for (int j = 0; j < C::NJ; ++j) {
+          const int col = bcol(j, 2 * t);
+          double2 v = *reinterpret_cast<const double2*>(cbuf + (col >> 4) * (C::BM * 128) + swz128_f64(r, col & 15));
+          v.x -= acc[i][j][2 * h];
+          v.y -= acc[i][j][2 * h + 1];
+          if (row < m) {
+            if (n0 + col + 1 < n) *reinterpret_cast<double2*>(p + col) = v;
+            else if (n0 + col < n) p[col] = v.x;
+          }
+        }
+      }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(cempty);
+    tile = next;
+  }
+  // leave no copy in flight behind: wait (bounded) for every issued stage's bytes
+  if (!ok && threadIdx.x == 0) {
+    for (int st = (issued > C::STAGES ? issued - C::STAGES : 0); st < issued; ++st)
+      mbar_wait(&full[st % C::STAGES], (st / C::STAGES) & 1u, status);
+    if (c_issued > 0) mbar_wait(cfull, (c_issued - 1) & 1u, status);
+  }
+}
+
+int dgemm_update_f64(int m, int n, int k, const double* a, int64_t lda, const double* b, int64_t ldb, double* c,
+                     int64_t ldc, const LeafMarks* marks, int most, int* counters, unsigned* status,
+                     cudaStream_t stream) {
+  CUtensorMap ta, tb, tc;
+  RM_TRY(make_tensor_map_2d(&ta, a, 8, k, m, lda * 8, 16, UpdateCfg::BM, true));
+  RM_TRY(make_tensor_map_2d(&tb, b, 8, n, k, ldb * 8, 16, 16, true));
+  RM_TRY(make_tensor_map_2d(&tc, c, 8, n, m, ldc * 8, 16, UpdateCfg::BM, true));  // checks C's alignment too
+  RM_TRY(smem_attribute(dgemm_update_kernel, kUpdateSmem));
+  const int sms = device_sm_count();
+  RM_CUDA_TRY(launch_dependent(dgemm_update_kernel, dim3(3 * sms), dim3(UpdateCfg::THREADS), kUpdateSmem,
+                               stream, ta, tb, tc, c, ldc, m, n, k, marks, 2 * sms + most, counters, status));
+  note_launch();
+  return RM_OK;
 }
 
 // ------------------------------------------------------------------ host side

@@ -6,18 +6,17 @@
 // right-looking in blocks of kOuter columns, so the trailing update is a rank-128 FP64
 // product (compute-bound on DMMA) instead of the rank-16..n/2 products of the recursion:
 //
-//   for each block of kOuter columns at J0:
+//   for each block of kOuter columns at J0 (getrf_block.cu):
 //     for each 32-column leaf at j0 inside it:
-//       panel_kernel     : pivot search, row swap, scale and rank-1 updates of the leaf,
-//                          rows spread over a cluster of up to 16 CTAs' shared memory
-//       swap_trsm_kernel : the leaf's swaps on the block's other columns, and
-//                          U = L^-1 A for the leaf's rows of the block's later columns
-//       dgemm            : the block's later columns below the leaf -= L21 U12
-//     swap_trsm_kernel   : the block's swaps on every column outside it, and perm
-//     invert_unit_lower_f64 : L11^-1 of the block's diagonal (4 CTAs, a 32-column block each)
-//     dgemm              : U12 = L11^-1 A12 (in place), then A22 -= L21 U12: the next
-//                          block's 128 columns first; for n >= 1024 the rest runs on a side
-//                          stream while the next block's leaves factor (look-ahead)
+//       leaf_kernel       : pivot search, scale and rank-1 updates of the leaf, the rows in the
+//                           registers of up to 16 CTAs (taller than 8192 rows: panel_kernel)
+//       leaf_tail_kernel  : the leaf's row moves on the block's other columns, U = L^-1 A for the
+//                           leaf's rows of the block's later columns, and those columns' update
+//     block_rows_kernel   : the block's row moves on every column outside it, and perm; U12 =
+//                           L11^-1 A12
+//     dgemm               : A22 -= L21 U12: the next block's 128 columns first; for n >= 1024 the
+//                           rest runs on a side stream while the next block's leaves factor
+//                           (look-ahead)
 //
 // The pivot rule is the reference's `largest` (factor.rs:476): the first row of greatest
 // magnitude, NaN never chosen, the diagonal itself when every candidate is NaN; a zero
@@ -28,61 +27,18 @@
 #include <mutex>
 #include <vector>
 
+#include "getrf_block.cuh"
+#include "rm_cluster.cuh"
 #include "rm_internal.h"
+#include "short_pivot.cuh"
 
 namespace rm {
 
-constexpr int kLeaf = 32;         // columns of a panel leaf
-constexpr int kOuter = 128;       // columns of an outer block (the trailing update's rank)
 constexpr int kPanelThreads = 256;
 constexpr int kPanelWarps = kPanelThreads / 32;
 constexpr int kPanelStride = kLeaf + 1;  // shared row stride (odd: conflict-free column reads)
 constexpr int kMaxCluster = 16;
 constexpr int kPanelSmemBudget = 200 * 1024;
-
-// ------------------------------------------------------------------ cluster helpers
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t cluster_nctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t map_rank(const void* p, uint32_t rank) {
-  uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
-  return a;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void st_cluster(uint32_t a, double v) {
-  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
-}
-__device__ __forceinline__ void st_cluster(uint32_t a, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
-}
-__device__ __forceinline__ void st_cluster(uint32_t a, int v) {
-  asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-}
-__device__ __forceinline__ double ld_cluster_f64(uint32_t a) {
-  double v;
-  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ float ld_cluster_f32(uint32_t a) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
-  return v;
-}
-template <typename T>
-__device__ __forceinline__ T ld_cluster(uint32_t a) {
-  if constexpr (sizeof(T) == 8) return ld_cluster_f64(a);
-  else return ld_cluster_f32(a);
-}
 
 template <typename T>
 __device__ __forceinline__ T min_normal() {
@@ -205,8 +161,8 @@ __global__ void __launch_bounds__(kPanelThreads)
       if (lane < jb) {
         T dv, pv;
         if (P > 1) {
-          dv = ld_cluster<T>(map_rank(&sh->diag[par][lane], owner_d));
-          pv = p == d ? dv : ld_cluster<T>(map_rank(&sh->cand[par][lane], owner_p));
+          dv = ld_cluster_f64(map_rank(&sh->diag[par][lane], owner_d));
+          pv = p == d ? dv : ld_cluster_f64(map_rank(&sh->cand[par][lane], owner_p));
         } else {
           dv = sh->diag[par][lane];
           pv = p == d ? dv : sh->cand[par][lane];
@@ -252,203 +208,6 @@ __global__ void __launch_bounds__(kPanelThreads)
   if (P > 1) cluster_sync_all();  // no CTA leaves while a peer may still read its memory
 }
 
-// ------------------------------------------------------------------ short leaves in one CTA
-// A leaf whose rows (M = n - j0 <= 768) fit one CTA: a thread per row, the leaf in shared
-// memory, factored in sub-leaves of 8 columns. Rows do not move while the leaf is factored:
-// each thread keeps its row's current position (relative to j0), a swap of positions d and p
-// only exchanges the two threads' positions, and at the end every row is stored at its final
-// position, which is where the explicit swaps of panel_kernel would have put it.
-//
-// Per sub-leaf, each thread holds its row's 8 items in registers and each column costs one CTA
-// barrier: a candidate's key is its magnitude's bits + 1 (0 for NaN and for rows already
-// chosen); each warp finds its largest key and, among equal keys, the lowest position (a
-// redux.sync of the keys' high words; when several lanes share the largest high word, two
-// more for the low words and the positions); its winner posts its sub-leaf row, position, key
-// and reciprocal (every candidate forms its reciprocal while the reduction runs); after the
-// barrier every warp reduces the posts the same way and reads the winning row. When every
-// candidate is NaN the pivot is the diagonal's row (factor.rs:476), posted after a second
-// barrier. After the sub-leaf, its pivot rows' later columns are solved against their unit
-// lower triangle (a thread per column) and the rows still unchosen take the rank-8 update.
-//
-// The arithmetic on every item is panel_kernel's: the same reciprocal, and per item the same
-// fma per pivot column in the same order (the deferred update applies the sub-leaf's columns
-// one fma at a time in column order; a zero pivot's column is skipped, as panel_kernel skips
-// it), so the results are the same bits. The sub-leaf loop is not unrolled: the kernel's code
-// stays in the instruction cache (a leaf fully unrolled over 32 columns was bound by
-// instruction fetch).
-constexpr int kShortLeafMaxRows = 768;
-constexpr int kShortWarps = kShortLeafMaxRows / 32;
-constexpr int kSub = 8;
-constexpr int kShortStride = kLeaf + 1;  // doubles per row in shared memory
-
-struct alignas(16) ShortPost {
-  double row[kSub];
-  unsigned long long key;
-  double rcp;
-  int pos;
-  int pad[3];
-};
-
-struct ShortShared {
-  ShortPost post[2][kShortWarps + 1];  // a post per warp, and the diagonal's row
-  double ub[kSub][kLeaf];              // the sub-leaf's pivot rows, later columns (U12)
-  int pv[kSub];                        // the thread (row) of each pivot of the sub-leaf
-  int pos[kShortLeafMaxRows];          // final positions
-};
-
-constexpr size_t short_leaf_smem(int rows) {
-  return (sizeof(ShortShared) + 15) / 16 * 16 + (size_t)rows * kShortStride * sizeof(double);
-}
-
-// The lane holding the warp's largest key, the lowest position among equal keys; `zero` when
-// every key is 0.
-__device__ __forceinline__ int short_reduce(unsigned long long key, unsigned pos, bool& zero) {
-  const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
-  const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
-  const unsigned top = __ballot_sync(0xffffffffu, hi == mhi);
-  zero = false;
-  if (__popc(top) == 1) return __ffs(top) - 1;  // mhi > 0 here: at most one lane holds a key of 0
-  const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
-  const bool tie = hi == mhi && lo == mlo;
-  const unsigned pmin = __reduce_min_sync(0xffffffffu, tie ? pos : 0xffffffffu);
-  zero = mhi == 0u && mlo == 0u;
-  return __ffs(__ballot_sync(0xffffffffu, tie && pos == pmin)) - 1;
-}
-
-// 1 / pivot as the cluster panel forms it (0 for a subnormal pivot, which is divided by)
-__device__ __forceinline__ double short_rcp(double pv) {
-  return fabs(pv) < 2.2250738585072014e-308 ? 0.0 : __drcp_rn(pv);
-}
-
-__device__ __forceinline__ void short_post(ShortPost& post, const double (&p)[kSub], int i, int pos,
-                                           unsigned long long key, double rcp) {
-  double2* dst = reinterpret_cast<double2*>(post.row);
-#pragma unroll
-  for (int q = i / 2; q < kSub / 2; ++q) dst[q] = make_double2(p[2 * q], p[2 * q + 1]);
-  post.rcp = rcp;
-  post.key = key;
-  post.pos = pos;
-}
-
-__global__ void __launch_bounds__(kShortLeafMaxRows, 1)
-    short_leaf_kernel(double* __restrict__ w, int64_t ldw, int n, int j0, int jb, int64_t* __restrict__ ipiv) {
-  extern __shared__ __align__(16) uint8_t smem[];
-  ShortShared& sh = *reinterpret_cast<ShortShared*>(smem);
-  double* S = reinterpret_cast<double*>(smem + (sizeof(ShortShared) + 15) / 16 * 16);
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  const int warps = blockDim.x >> 5;
-  const int M = n - j0;
-  griddep_launch_dependents();
-  griddep_wait();  // the kernel before this one in the stream has completed
-  // the leaf into shared memory: a warp per row, lanes along it (coalesced)
-  for (int r = warp; r < M; r += warps)
-    if (lane < jb) S[r * kShortStride + lane] = w[(int64_t)(j0 + r) * ldw + j0 + lane];
-  __syncthreads();
-  double* row = S + t * kShortStride;
-  int pos = t < M ? t : INT_MAX;  // the row's current position; threads past M take no part
-  bool active = t < M;
-#pragma unroll 1
-  for (int c0 = 0; c0 < jb; c0 += kSub) {
-    double p[kSub];
-#pragma unroll
-    for (int i = 0; i < kSub; ++i) p[i] = (t < M && c0 + i < jb) ? row[c0 + i] : 0.0;
-    unsigned skip = 0;  // the sub-leaf's columns whose pivot was zero (left unreduced)
-#pragma unroll
-    for (int i = 0; i < kSub; ++i) {
-      const int c = c0 + i;
-      if (c >= jb) break;
-      ShortPost* pp = sh.post[c & 1];
-      const double a = fabs(p[i]);
-      const unsigned long long key =
-          (active && a == a) ? (unsigned long long)__double_as_longlong(a) + 1ull : 0ull;
-      const double myr = short_rcp(p[i]);
-      bool none;
-      const int wl = short_reduce(key, (unsigned)pos, none);
-      if (lane == wl) short_post(pp[warp], p, i, pos, key, myr);
-      __syncthreads();
-      // every warp reduces the posts: the largest key, the lowest position among equals
-      const unsigned long long k2 = lane < warps ? pp[lane].key : 0ull;
-      const unsigned p2 = lane < warps ? (unsigned)pp[lane].pos : 0xffffffffu;
-      const int bw = short_reduce(k2, p2, none);
-      const ShortPost* win = &pp[bw];
-      if (none) {  // every candidate is NaN: the diagonal's row is the pivot row
-        if (pos == c) short_post(pp[kShortWarps], p, i, pos, 0ull, myr);
-        __syncthreads();
-        win = &pp[kShortWarps];
-      }
-      const int pr = win->pos;
-      const double pivot = win->row[i];
-      const double r = win->rcp;
-      if (pos == pr) {
-        active = false;
-        pos = c;
-        sh.pv[i] = t;
-      } else if (pos == c) {
-        pos = pr;
-      }
-      if (t == 0) ipiv[j0 + c] = j0 + pr;
-      if (pivot == 0.0) skip |= 1u << i;
-      if (active && pivot != 0.0) {
-        const bool sub = fabs(pivot) < 2.2250738585072014e-308;
-        double l = p[i];
-        l = sub ? l / pivot : l * r;
-        p[i] = l;
-        const double2* prow = reinterpret_cast<const double2*>(win->row);
-#pragma unroll
-        for (int q = (i + 1) / 2; q < kSub / 2; ++q) {
-          const double2 u = prow[q];
-          if (2 * q > i) p[2 * q] = fma(l, -u.x, p[2 * q]);
-          if (2 * q + 1 > i) p[2 * q + 1] = fma(l, -u.y, p[2 * q + 1]);
-        }
-      }
-    }
-    if (t < M) {
-#pragma unroll
-      for (int i = 0; i < kSub; ++i)
-        if (c0 + i < jb) row[c0 + i] = p[i];
-    }
-    const int rc0 = c0 + kSub, rcols = jb - rc0;
-    if (rcols <= 0) break;
-    __syncthreads();
-    // U12: the sub-leaf's pivot rows, later columns, against their unit lower triangle; a
-    // thread per column, the same fmas in the same order as the rank-1 updates
-    if (t < rcols) {
-      double u[kSub];
-#pragma unroll
-      for (int k = 0; k < kSub; ++k) u[k] = S[sh.pv[k] * kShortStride + rc0 + t];
-#pragma unroll
-      for (int k = 1; k < kSub; ++k) {
-        const double* lrow = S + sh.pv[k] * kShortStride + c0;
-#pragma unroll
-        for (int q = 0; q < k; ++q)
-          if (!((skip >> q) & 1u)) u[k] = fma(lrow[q], -u[q], u[k]);
-      }
-#pragma unroll
-      for (int k = 0; k < kSub; ++k) {
-        S[sh.pv[k] * kShortStride + rc0 + t] = u[k];
-        sh.ub[k][t] = u[k];
-      }
-    }
-    __syncthreads();
-    // the rows still unchosen: later columns, one fma per pivot column in column order
-    if (active) {
-      for (int j = 0; j < rcols; ++j) {
-        double x = row[rc0 + j];
-#pragma unroll
-        for (int k = 0; k < kSub; ++k)
-          if (!((skip >> k) & 1u)) x = fma(p[k], -sh.ub[k][j], x);
-        row[rc0 + j] = x;
-      }
-    }
-    __syncthreads();
-  }
-  // the leaf back, every row at its final position: a warp per row, lanes along it
-  if (t < M) sh.pos[t] = pos;
-  __syncthreads();
-  for (int r2 = warp; r2 < M; r2 += warps)
-    if (lane < jb) w[(int64_t)(j0 + sh.pos[r2]) * ldw + j0 + lane] = S[r2 * kShortStride + lane];
-}
-
 // ------------------------------------------------------------------ a whole matrix in a cluster
 // n <= 256: the whole matrix lives in the shared memory of one cluster of C <= 8 CTAs (a power
 // of two, at most 32 rows per CTA; 66 KB per CTA at n = 256) and is factored in one launch,
@@ -461,7 +220,7 @@ __global__ void __launch_bounds__(kShortLeafMaxRows, 1)
 // CTA's shared memory), so at n = 384..512 the blocked path is faster and keeps those sizes.
 //
 // Rows do not move. Every warp of a CTA tracks the positions of the CTA's rows (lane = row), so
-// a pivot choice only exchanges two positions, as in short_leaf_kernel; at the end each row is
+// a pivot choice only exchanges two positions, as in leaf_kernel; at the end each row is
 // stored at its final position. Per pivot column j, after the barrier that publishes column j's
 // candidates:
 //   - every warp reduces the C posts (largest key, lowest position among equals; when every
@@ -493,10 +252,6 @@ struct alignas(16) ClusterPost {
 struct ClusterLuShared {
   ClusterPost post[2][kMaxCluster];  // [column parity][posting CTA]
 };
-
-__device__ __forceinline__ void st_cluster_u64(uint32_t a, unsigned long long v) {
-  asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
-}
 
 // Warp 0 of each CTA: the CTA's candidate for column `col` (y = this lane's row's item) and, if
 // the CTA holds it, the row at position `col`, stored into slot `slot` of every CTA's posts.
@@ -763,125 +518,6 @@ int small_solve_f64(const double* w, int64_t ldw, bool colmajor, int64_t n, cons
   return RM_OK;
 }
 
-// ------------------------------------------------------------------ swaps + unit-lower solve
-constexpr int kSwapCols = 16;      // columns per CTA
-constexpr int kSwapThreads = 256;
-constexpr int kMaxSwaps = kOuter;  // pivots applied by one launch
-
-// Applies the swaps ipiv[j0..j0+jb) in order to the columns [lo1,hi1) and [lo2,hi2) of W.
-// With trsm_lo < trsm_hi, rows j0..j0+jb-1 of the columns in that range are then replaced
-// by L^-1 times them, L the unit lower triangle of W[j0.., j0..] (jb <= kLeaf). Block 0
-// also applies the swaps to perm when perm is not NULL.
-template <typename T>
-__global__ void __launch_bounds__(kSwapThreads)
-    swap_trsm_kernel(T* __restrict__ w, int64_t ldw, int j0, int jb, const int64_t* __restrict__ ipiv, int lo1,
-                     int hi1, int lo2, int hi2, int trsm_lo, int trsm_hi, int64_t* __restrict__ perm) {
-  __shared__ int pos[2 * kMaxSwaps], src[2 * kMaxSwaps];
-  __shared__ int count;
-  __shared__ T buf[2 * kMaxSwaps][kSwapCols + 1];
-  __shared__ T lblk[kLeaf][kLeaf + 1];
-  __shared__ int ipv[kMaxSwaps];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  griddep_launch_dependents();
-  griddep_wait();  // the kernel before this one in the stream has completed
-  // the swaps' targets, all at once (the loop below is sequential over them)
-  for (int q = tid; q < jb; q += kSwapThreads) ipv[q] = (int)ipiv[j0 + q];
-  __syncthreads();
-
-  // ---- the net effect of the swaps: row pos[e] receives the old row src[e]
-  if (warp == 0) {
-    for (int q = lane; q < jb; q += 32) pos[q] = src[q] = j0 + q;
-    int cntE = jb;
-    for (int i = 0; i < jb; ++i) {
-      const int d = j0 + i, p = ipv[i];
-      if (p == d) continue;
-      int e;
-      if (p < j0 + jb) {
-        e = p - j0;
-      } else {
-        e = -1;
-        for (int b = jb; b < cntE && e < 0; b += 32) {
-          const unsigned hit = __ballot_sync(0xffffffffu, b + lane < cntE && pos[b + lane] == p);
-          if (hit) e = b + __ffs(hit) - 1;
-        }
-        if (e < 0) {
-          e = cntE;
-          if (lane == 0) pos[e] = src[e] = p;
-          ++cntE;
-        }
-        __syncwarp();
-      }
-      if (lane == 0) {
-        const int t = src[i];
-        src[i] = src[e];
-        src[e] = t;
-      }
-      __syncwarp();
-    }
-    if (lane == 0) count = cntE;
-  }
-  __syncthreads();
-  const int E = count;
-
-  // ---- the columns of this CTA
-  const int chunks1 = (hi1 - lo1 + kSwapCols - 1) / kSwapCols;
-  int c0, c1;
-  if ((int)blockIdx.x < chunks1) {
-    c0 = lo1 + blockIdx.x * kSwapCols;
-    c1 = min(c0 + kSwapCols, hi1);
-  } else {
-    c0 = lo2 + (blockIdx.x - chunks1) * kSwapCols;
-    c1 = min(c0 + kSwapCols, hi2);
-  }
-  const int width = c1 - c0;
-
-  if (width > 0) {
-    for (int e = tid; e < E * kSwapCols; e += kSwapThreads) {
-      const int r = e / kSwapCols, cc = e - r * kSwapCols;
-      if (cc < width) buf[r][cc] = w[(int64_t)src[r] * ldw + c0 + cc];
-    }
-  }
-  const bool solve = width > 0 && trsm_lo < trsm_hi && c0 >= trsm_lo && c1 <= trsm_hi;
-  if (solve)
-    for (int e = tid; e < jb * kLeaf; e += kSwapThreads) {
-      const int r = e / kLeaf, cc = e - r * kLeaf;
-      lblk[r][cc] = cc < jb ? w[(int64_t)(j0 + r) * ldw + j0 + cc] : T(0);
-    }
-  __syncthreads();
-  if (solve) {
-    // one warp per column: lane r holds row r; row i is final once rows < i are removed
-    for (int cc = warp; cc < width; cc += kSwapThreads / 32) {
-      T x = lane < jb ? buf[lane][cc] : T(0);
-      for (int i = 0; i < jb; ++i) {
-        const T xi = __shfl_sync(0xffffffffu, x, i);
-        if (lane > i && lane < jb) x = fma(-lblk[lane][i], xi, x);
-      }
-      if (lane < jb) buf[lane][cc] = x;
-    }
-    __syncthreads();
-  }
-  if (width > 0) {
-    for (int e = tid; e < E * kSwapCols; e += kSwapThreads) {
-      const int r = e / kSwapCols, cc = e - r * kSwapCols;
-      if (cc < width && (pos[r] != src[r] || (solve && r < jb))) w[(int64_t)pos[r] * ldw + c0 + cc] = buf[r][cc];
-    }
-  }
-  if (perm != nullptr && blockIdx.x == 0) {
-    int64_t v[(2 * kMaxSwaps + kSwapThreads - 1) / kSwapThreads];
-#pragma unroll
-    for (int s = 0; s < (int)(sizeof(v) / sizeof(v[0])); ++s) {
-      const int e = tid + s * kSwapThreads;
-      v[s] = e < E ? perm[src[e]] : 0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int s = 0; s < (int)(sizeof(v) / sizeof(v[0])); ++s) {
-      const int e = tid + s * kSwapThreads;
-      if (e < E) perm[pos[e]] = v[s];
-    }
-  }
-}
-
 // ------------------------------------------------------------------ driver
 
 // The largest cluster (<= kMaxCluster CTAs of kPanelSmemBudget bytes) this device can place.
@@ -1003,15 +639,6 @@ static int launch_cluster_lu(double* w, int64_t ldw, int n, int64_t* ipiv, int64
 template <typename T>
 static int launch_panel(T* w, int64_t ldw, int n, int j0, int jb, int64_t* ipiv, cudaStream_t stream) {
   const int M = n - j0;
-  if constexpr (sizeof(T) == 8) {
-    if (M <= kShortLeafMaxRows) {  // one CTA, a thread per row
-      RM_TRY(smem_attribute(short_leaf_kernel, short_leaf_smem(kShortLeafMaxRows)));
-      RM_CUDA_TRY(launch_dependent(short_leaf_kernel, dim3(1), dim3((M + 31) / 32 * 32), short_leaf_smem(M), stream, w,
-                                   ldw, n, j0, jb, ipiv));
-      note_launch();
-      return RM_OK;
-    }
-  }
   const size_t sh = (sizeof(PanelShared<T>) + 15) / 16 * 16;
   const int rows_cap = (int)((kPanelSmemBudget - sh) / (kPanelStride * sizeof(T)));
   const int pmax = panel_cluster_limit<T>();
@@ -1044,90 +671,22 @@ static int launch_panel(T* w, int64_t ldw, int n, int j0, int jb, int64_t* ipiv,
   return RM_OK;
 }
 
-template <typename T>
-static int launch_swap(T* w, int64_t ldw, int j0, int jb, const int64_t* ipiv, int lo1, int hi1, int lo2, int hi2,
-                       int trsm_lo, int trsm_hi, int64_t* perm, cudaStream_t stream) {
-  hi1 = max(hi1, lo1);
-  hi2 = max(hi2, lo2);
-  const int chunks = (hi1 - lo1 + kSwapCols - 1) / kSwapCols + (hi2 - lo2 + kSwapCols - 1) / kSwapCols;
-  const int grid = max(chunks, perm ? 1 : 0);
-  if (grid == 0) return RM_OK;
-  RM_CUDA_TRY(launch_dependent(swap_trsm_kernel<T>, dim3(grid), dim3(kSwapThreads), 0, stream, w, ldw, j0, jb, ipiv, lo1,
-                               hi1, lo2, hi2, trsm_lo, trsm_hi, perm));
-  note_launch();
-  return RM_OK;
-}
-
-// L11^-1 of the unit lower triangle of the nb x nb diagonal block at (j0, j0) (row-major,
-// ld kOuter, zeros above the diagonal; identity beyond nb), a 32-column block of it per CTA
-// (4 CTAs), everything in shared memory: CTA a forms X_aa = D_a^-1 and then, block row by block
-// row, X_ba = -D_b^-1 sum_{c=a..b-1} L_bc X_ca; the diagonal blocks' inverses D_b^-1 first, a
-// warp each, a lane per column (forward substitution).
-constexpr int kInvS = kOuter + 1;
-constexpr size_t kInv64Smem = ((size_t)kOuter * kInvS + (size_t)(4 * kLeaf + kOuter + kLeaf) * (kLeaf + 1)) *
-                              sizeof(double);
-
-__global__ void __launch_bounds__(256) invert_unit_lower_f64_kernel(const double* __restrict__ w, int64_t ldw, int j0,
-                                                                    int nb, double* __restrict__ out) {
-  extern __shared__ __align__(16) uint8_t smraw[];
-  double(*M)[kInvS] = reinterpret_cast<double(*)[kInvS]>(smraw);
-  double(*Y)[kLeaf + 1] = reinterpret_cast<double(*)[kLeaf + 1]>(smraw + (size_t)kOuter * kInvS * sizeof(double));
-  double(*X)[kLeaf + 1] = Y + 4 * kLeaf;  // the column block, rows 0..127
-  double(*Tq)[kLeaf + 1] = X + kOuter;     // 32 x 33
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int ab = blockIdx.x, a0 = kLeaf * ab;
-  const double* l = w + (int64_t)j0 * ldw + j0;
-  griddep_launch_dependents();
-  griddep_wait();  // the kernel before this one in the stream has completed
-  // L from row and column a0 on (strictly lower part; unit diagonal implied)
-  for (int i = a0 + warp; i < kOuter; i += 8)
-    for (int k = a0 + lane; k < kOuter; k += 32) M[i][k] = (i < nb && k < nb && k < i) ? l[(int64_t)i * ldw + k] : 0.0;
-  __syncthreads();
-  if (warp < 4 - ab) {  // Y_b = D_b^-1, b = ab + warp
-    const int b0 = a0 + kLeaf * warp;
-    double x[kLeaf];
-#pragma unroll
-    for (int i = 0; i < kLeaf; ++i) {
-      double acc = i == lane ? 1.0 : 0.0;
-#pragma unroll
-      for (int k2 = 0; k2 < i; ++k2) acc = fma(-M[b0 + i][b0 + k2], x[k2], acc);
-      x[i] = i < lane ? 0.0 : acc;
-    }
-#pragma unroll
-    for (int i = 0; i < kLeaf; ++i) Y[b0 + i][lane] = x[i];
-  }
-  __syncthreads();
-  for (int e = tid; e < kLeaf * kLeaf; e += 256) X[a0 + (e >> 5)][e & 31] = Y[a0 + (e >> 5)][e & 31];
-  __syncthreads();
-  const int ti = tid >> 4, tj = tid & 15;  // rows ti, ti + 16 and columns tj, tj + 16 of a 32 x 32 block
-  for (int b = ab + 1; b < 4; ++b) {
-    const int r0 = kLeaf * b + ti, r1 = r0 + 16;
-    double t00 = 0.0, t01 = 0.0, t10 = 0.0, t11 = 0.0;
-#pragma unroll 4
-    for (int k = a0; k < kLeaf * b; ++k) {
-      const double m0 = M[r0][k], m1 = M[r1][k], x0 = X[k][tj], x1 = X[k][tj + 16];
-      t00 = fma(m0, x0, t00), t01 = fma(m0, x1, t01), t10 = fma(m1, x0, t10), t11 = fma(m1, x1, t11);
-    }
-    Tq[ti][tj] = t00, Tq[ti][tj + 16] = t01, Tq[ti + 16][tj] = t10, Tq[ti + 16][tj + 16] = t11;
-    __syncthreads();
-    t00 = t01 = t10 = t11 = 0.0;
-#pragma unroll 4
-    for (int k2 = 0; k2 < kLeaf; ++k2) {
-      const double y0 = Y[r0][k2], y1 = Y[r1][k2], u0 = Tq[k2][tj], u1 = Tq[k2][tj + 16];
-      t00 = fma(y0, u0, t00), t01 = fma(y0, u1, t01), t10 = fma(y1, u0, t10), t11 = fma(y1, u1, t11);
-    }
-    X[r0][tj] = -t00, X[r0][tj + 16] = -t01, X[r1][tj] = -t10, X[r1][tj + 16] = -t11;
-    __syncthreads();
-  }
-  for (int rr = warp; rr < kOuter; rr += 8) out[rr * kOuter + a0 + lane] = rr >= a0 ? X[rr][lane] : 0.0;
-}
-
 __global__ void iota_kernel(int64_t* perm, int64_t n) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     perm[i] = i;
 }
 
-size_t getrf_f64_scratch_bytes(int64_t n) { return (size_t)kOuter * kOuter * sizeof(double) + 256; }
+namespace {
+struct GetrfScratch {
+  BlockScratch block[2];         // by the block's parity: the side stream still reads the last one's
+  LeafMarks marks;
+};
+}  // namespace
+
+// the look-ahead's counters follow: two ints per block
+size_t getrf_f64_scratch_bytes(int64_t n) {
+  return sizeof(GetrfScratch) + (size_t)((n + kOuter - 1) / kOuter) * 2 * sizeof(int);
+}
 
 namespace {
 // The look-ahead's streams: the critical chain (hp) at the device's highest stream priority, the
@@ -1135,20 +694,20 @@ namespace {
 // SMs first as the update's tiles finish. Released on return (queued work completes first).
 struct F64LookAhead {
   cudaStream_t hp = nullptr, side = nullptr;
-  cudaEvent_t next_done = nullptr, rest_done = nullptr, entry = nullptr;
+  cudaEvent_t leaves_done = nullptr, rest_done = nullptr, entry = nullptr;
   int open() {
     int least = 0, greatest = 0;
     RM_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest));
     RM_CUDA_TRY(cudaStreamCreateWithPriority(&hp, cudaStreamNonBlocking, greatest));
     RM_CUDA_TRY(cudaStreamCreateWithPriority(&side, cudaStreamNonBlocking, least));
-    RM_CUDA_TRY(cudaEventCreateWithFlags(&next_done, cudaEventDisableTiming));
+    RM_CUDA_TRY(cudaEventCreateWithFlags(&leaves_done, cudaEventDisableTiming));
     RM_CUDA_TRY(cudaEventCreateWithFlags(&rest_done, cudaEventDisableTiming));
     RM_CUDA_TRY(cudaEventCreateWithFlags(&entry, cudaEventDisableTiming));
     RM_CUDA_TRY(cudaEventRecord(rest_done, side));  // complete at first, so the first wait passes
     return RM_OK;
   }
   ~F64LookAhead() {
-    if (next_done) cudaEventDestroy(next_done);
+    if (leaves_done) cudaEventDestroy(leaves_done);
     if (rest_done) cudaEventDestroy(rest_done);
     if (entry) cudaEventDestroy(entry);
     if (hp) cudaStreamDestroy(hp);
@@ -1163,17 +722,26 @@ int getrf_f64(double* w, int64_t ldw, int64_t n64, int64_t* ipiv, int64_t* perm,
   if (n64 > INT32_MAX / 2) return RM_BAD_ARG;
   const int n = (int)n64;
   if (n <= kClusterLuMax && cluster_lu_ok()) return launch_cluster_lu(w, ldw, n, ipiv, perm, caller);
-  double* linv = reinterpret_cast<double*>(scratch);
+  GetrfScratch* gs = reinterpret_cast<GetrfScratch*>(scratch);
+  int* counters = reinterpret_cast<int*>(gs + 1);
   iota_kernel<<<std::max(1, std::min(n / 256 + 1, 1024)), 256, 0, caller>>>(perm, n);
   RM_LAUNCHED();
-  // Look-ahead (n >= 1024): each trailing update does the next block's 128 columns first, on
-  // the chain's stream; the rest runs on a side stream while the next block's leaves factor.
-  // Only the block's row swaps on the columns right of it wait for that rest (it writes them).
-  RM_TRY(smem_attribute(invert_unit_lower_f64_kernel, kInv64Smem));
+  // Look-ahead (n >= 1024): the chain's stream does only what the next block's leaves wait for: the
+  // block's rows and the trailing update of the next block's 128 columns. The same on all other
+  // columns, and the row moves of the columns left of the block, run on a side stream while the
+  // next block's leaves factor; the chain waits for the side stream before it touches columns that
+  // the side's update wrote.
+  //
+  // The leaves' clusters need up to 16 free SMs of one GPC at once, which a trailing update that
+  // fills the GPU never leaves: with a plain grid for it, chain and update ran one after the other
+  // (n = 8192: 34 ms, the chain alone 20, the update alone 11). So the update is a persistent grid
+  // whose CTAs do not stay on the SMs where the latest leaf ran.
   F64LookAhead la;
   const bool ahead = n >= 1024;
   cudaStream_t stream = caller;
   if (ahead) {
+    RM_CUDA_TRY(cudaMemsetAsync(&gs->marks, 0, sizeof gs->marks, caller));
+    RM_CUDA_TRY(cudaMemsetAsync(counters, 0, (size_t)((n + kOuter - 1) / kOuter) * 2 * sizeof(int), caller));
     RM_TRY(la.open());
     RM_CUDA_TRY(cudaEventRecord(la.entry, caller));
     RM_CUDA_TRY(cudaStreamWaitEvent(la.hp, la.entry, 0));
@@ -1182,46 +750,47 @@ int getrf_f64(double* w, int64_t ldw, int64_t n64, int64_t* ipiv, int64_t* perm,
   for (int J0 = 0; J0 < n; J0 += kOuter) {
     const int nb = std::min(kOuter, n - J0);
     const int J1 = J0 + nb;
+    BlockScratch* bs = &gs->block[J0 / kOuter & 1];
     for (int j0 = J0; j0 < J1; j0 += kLeaf) {
       const int jb = std::min(kLeaf, J1 - j0);
-      RM_TRY(launch_panel<double>(w, ldw, n, j0, jb, ipiv, stream));
-      // the leaf's swaps on the block's other columns; solve for its rows of later columns
-      RM_TRY(launch_swap<double>(w, ldw, j0, jb, ipiv, J0, j0, j0 + jb, J1, j0 + jb, J1, nullptr, stream));
-      if (j0 + jb < J1 && j0 + jb < n) {
-        const int64_t rows = n - (j0 + jb), cols = J1 - (j0 + jb);
-        RM_TRY(dgemm_device(false, false, rows, cols, jb, -1.0, w + (int64_t)(j0 + jb) * ldw + j0, ldw,
-                            w + (int64_t)j0 * ldw + j0 + jb, ldw, 1.0, w + (int64_t)(j0 + jb) * ldw + j0 + jb, ldw,
-                            status, stream));
+      if (n - j0 <= kLeafMaxRows) {
+        RM_TRY(leaf_f64(w, ldw, n, j0, jb, J0, J1, bs, ahead ? &gs->marks : nullptr, status, stream));
+      } else {
+        RM_TRY(launch_panel<double>(w, ldw, n, j0, jb, ipiv, stream));
+        RM_TRY(leaf_moves_f64(w, ldw, j0, jb, J0, J1, ipiv, bs, stream));
       }
+      if (j0 + jb < J1) RM_TRY(leaf_tail_f64(w, ldw, n, j0, J0, J1, bs, stream));
     }
-    // the block's swaps on every other column, and the row permutation (after the rest of the
-    // last trailing update, which writes the columns right of this block)
-    if (ahead && J0 > 0) RM_CUDA_TRY(cudaStreamWaitEvent(stream, la.rest_done, 0));
-    RM_TRY(launch_swap<double>(w, ldw, J0, nb, ipiv, 0, J0, J1, n, 0, 0, perm, stream));
-    if (J1 < n) {
-      RM_CUDA_TRY(launch_dependent(invert_unit_lower_f64_kernel, dim3(kOuter / kLeaf), dim3(256), kInv64Smem, stream,
-                                   (const double*)w, ldw, J0, nb, linv));
-      note_launch();
-      double* a12 = w + (int64_t)J0 * ldw + J1;
-      RM_TRY(dgemm_device(false, false, nb, n - J1, nb, 1.0, linv, kOuter, a12, ldw, 0.0, a12, ldw, status, stream,
-                          /*force_wide_m=*/true));
-      const double* l21 = w + (int64_t)J1 * ldw + J0;
-      double* a22 = w + (int64_t)J1 * ldw + J1;
-      const int rest = n - J1;
-      if (!ahead) {
+    const double* a12 = w + (int64_t)J0 * ldw + J1;
+    const double* l21 = w + (int64_t)J1 * ldw + J0;
+    double* a22 = w + (int64_t)J1 * ldw + J1;
+    const int rest = n - J1;
+    if (!ahead) {
+      RM_TRY(block_rows_f64(w, ldw, J0, nb, true, J1, n, bs, perm, stream));
+      if (rest > 0)
         RM_TRY(dgemm_device(false, false, rest, rest, nb, -1.0, l21, ldw, a12, ldw, 1.0, a22, ldw, status, stream));
-        continue;
-      }
-      const int nn = std::min(kOuter, rest);
+      continue;
+    }
+    // the side stream needs the leaves, not the chain's part of the block's end
+    const int nn = std::min(kOuter, rest);
+    RM_CUDA_TRY(cudaEventRecord(la.leaves_done, stream));
+    RM_CUDA_TRY(cudaStreamWaitEvent(la.side, la.leaves_done, 0));
+    if (nn > 0) {
+      if (J0 > 0) RM_CUDA_TRY(cudaStreamWaitEvent(stream, la.rest_done, 0));
+      RM_TRY(block_rows_f64(w, ldw, J0, nb, false, J1, J1 + nn, bs, nullptr, stream));
       RM_TRY(dgemm_device(false, false, rest, nn, nb, -1.0, l21, ldw, a12, ldw, 1.0, a22, ldw, status, stream));
-      if (rest > nn) {
-        RM_CUDA_TRY(cudaEventRecord(la.next_done, stream));
-        RM_CUDA_TRY(cudaStreamWaitEvent(la.side, la.next_done, 0));
+    }
+    RM_TRY(block_rows_f64(w, ldw, J0, nb, true, J1 + nn, n, bs, perm, la.side));
+    if (rest > nn) {
+      const int64_t tiles = (int64_t)((rest + 127) / 128) * ((rest - nn + 127) / 128);
+      if (tiles >= device_sm_count())
+        RM_TRY(dgemm_update_f64(rest, rest - nn, nb, l21, ldw, a12 + nn, ldw, a22 + nn, ldw, &gs->marks, kMaxCluster,
+                                counters + 2 * (J0 / kOuter), status, la.side));
+      else
         RM_TRY(dgemm_device(false, false, rest, rest - nn, nb, -1.0, l21, ldw, a12 + nn, ldw, 1.0, a22 + nn, ldw, status,
                             la.side));
-        RM_CUDA_TRY(cudaEventRecord(la.rest_done, la.side));
-      }
     }
+    RM_CUDA_TRY(cudaEventRecord(la.rest_done, la.side));
   }
   if (ahead) {
     RM_CUDA_TRY(cudaStreamWaitEvent(stream, la.rest_done, 0));
