@@ -13,6 +13,7 @@
 // half-warp touches 16 distinct 8-byte bank pairs under the 128-byte swizzle.
 #include <climits>
 
+#include "dgemm_lower.cuh"
 #include "getrf_block.cuh"
 #include "rm_internal.h"
 
@@ -51,8 +52,9 @@ __device__ __forceinline__ uint32_t tile_off(uint32_t mn, uint32_t k) {
 template <class C>
 __global__ void __launch_bounds__(C::THREADS, 1)
     dgemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                 double* __restrict__ c, int64_t ldc, int m, int n, int k, double alpha, double beta,
+                 double* __restrict__ c, int64_t ldc, int m, int n, int k, double alpha, double beta, bool lower,
                  unsigned* status) {
+  if (lower && (int)(blockIdx.x * C::BN) >= (int)(blockIdx.y + 1) * C::BM) return;  // strictly above the diagonal
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::STAGES * C::STAGE_BYTES);
@@ -410,7 +412,7 @@ int dgemm_update_f64(int m, int n, int k, const double* a, int64_t lda, const do
 
 template <class C>
 static int launch_cfg(const double* a, int64_t lda, const double* b, int64_t ldb, double* c, int64_t ldc, int m,
-                      int n, int k, double alpha, double beta, unsigned* status, cudaStream_t stream) {
+                      int n, int k, double alpha, double beta, unsigned* status, cudaStream_t stream, bool lower = false) {
   CUtensorMap ta, tb;
   // A: op(A) is m x k. Not transposed: stored m rows of k; transposed: k rows of m.
   if (!C::TA) {
@@ -426,7 +428,7 @@ static int launch_cfg(const double* a, int64_t lda, const double* b, int64_t ldb
   RM_TRY(smem_attribute(dgemm_kernel<C>, C::SMEM));
   dim3 grid((n + C::BN - 1) / C::BN, (m + C::BM - 1) / C::BM);
   RM_CUDA_TRY(launch_dependent(dgemm_kernel<C>, grid, dim3(C::THREADS), C::SMEM, stream, ta, tb, c, ldc, m, n, k, alpha,
-                               beta, status));
+                               beta, lower, status));
   note_launch();
   return RM_OK;
 }
@@ -455,6 +457,18 @@ int dgemm_device(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha
   }
   if (tb) return launch_t<false, true>(a, lda, b, ldb, c, ldc, (int)m, (int)n, (int)k, alpha, beta, status, stream, wide);
   return launch_t<false, false>(a, lda, b, ldb, c, ldc, (int)m, (int)n, (int)k, alpha, beta, status, stream, wide);
+}
+
+int dgemm_lower_device(int64_t n, int64_t k, double alpha, const double* a, int64_t lda, const double* b, int64_t ldb,
+                       double beta, double* c, int64_t ldc, unsigned* status, cudaStream_t stream) {
+  if (n == 0) return RM_OK;
+  if (n > INT32_MAX || k < 1 || k > INT32_MAX) return RM_BAD_ARG;
+  const int64_t t = (n + 127) / 128, big_tiles = t * (t + 1) / 2;
+  if (big_tiles >= device_sm_count())
+    return launch_cfg<DgemmCfg<128, 128, 64, 32, 4, false, true>>(a, lda, b, ldb, c, ldc, (int)n, (int)n, (int)k, alpha,
+                                                                  beta, status, stream, true);
+  return launch_cfg<DgemmCfg<64, 64, 32, 32, 4, false, true>>(a, lda, b, ldb, c, ldc, (int)n, (int)n, (int)k, alpha, beta,
+                                                              status, stream, true);
 }
 
 // C = beta*C (beta == 0 writes zeros), the reference's `scale` (linalg.rs:1000-1008).

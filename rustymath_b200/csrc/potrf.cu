@@ -5,18 +5,19 @@
 // factors blocks of cholesky_block(n) columns by recursive halving down to 16-column leaves,
 // then updates the rest with `gram` (the lower triangle of C - X X^T). Here, on a row-major
 // working copy W (ld a multiple of 32):
-//   - each 64-column diagonal block is factored column by column in one CTA's shared memory
-//     (sqrt of the pivot, the column below divided by it the way rustymath's `divide` does, the
-//     later columns of the block reduced by FMAs in column order), and the same CTA inverts L11;
-//   - the rows below it become L21 = A21 L11^-T through one float64 tensor-core GEMM (dgemm.cu);
-//   - the trailing matrix takes A22 -= L21 L21^T through another (the whole square is formed;
-//     only its lower triangle is read again).
+//   - each 64-column diagonal block is factored in one CTA's shared memory (sqrt of the pivot, the
+//     column below divided by it the way rustymath's `divide` does, the later columns of the block
+//     reduced by FMAs in column order), and the same CTA inverts L11;
+//   - the rows below it become L21 = A21 L11^-T in place through one float64 tensor-core GEMM
+//     (dgemm.cu);
+//   - the trailing matrix's lower triangle takes A22 -= L21 L21^T through another.
 // A pivot that is not > 0 (NaN included) marks the matrix not positive definite, as rustymath's
 // None; later blocks then work on whatever is left and their results are not used.
 // Stacks of small matrices (n <= 128) factor one matrix per CTA, entirely in shared memory, in
 // one launch; a matrix that is not positive definite gives NaN everywhere, as rustymath's stacks.
 #include <cfloat>
 
+#include "dgemm_lower.cuh"
 #include "rm_internal.h"
 
 namespace rm {
@@ -61,43 +62,148 @@ __device__ bool chol_in_smem(double* S, int lds, int nb) {
 // factored in shared memory and written back (lower triangle), and its inverse L11^-1 goes to
 // linv (row-major kPotrfBlock x kPotrfBlock, zeros above the diagonal and past nb). A block
 // that is not positive definite sets *notpd.
+//
+// The block is on the factorization's critical path and is bound by latency: 16 columns at a time, a
+// thread per row with its 16 items in registers, and per column one barrier of those two warps,
+// after which every thread forms the square root and its reciprocal for itself (~300 cycles a
+// column); the later columns take the 16 on DMMA, and the inverse is put together from the four
+// 16 x 16 diagonal blocks' inverses (a warp each) on DMMA. Column by column over the whole block
+// with two CTA barriers each, and the inverse as one chain per column, took 108 us a block.
+// Rows past nb are the identity's.
+constexpr int kPotrfSub = 16;
+constexpr int kPotrfLds = kPotrfBlock + 4;  // fragment loads hit 16 distinct 8-byte banks
+
+__device__ __forceinline__ void potrf_mma(double (&d)[4], const double (&a)[4], double b0, double b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b0), "d"(b1));
+}
+
 __global__ void __launch_bounds__(kPotrfThreads) potrf_diag_kernel(double* __restrict__ w, int64_t ld, int nb,
                                                                    double* __restrict__ linv, int* notpd) {
-  extern __shared__ double psm[];
-  constexpr int LDS = kPotrfBlock + 1;
+  extern __shared__ __align__(16) double psm[];
+  constexpr int LDS = kPotrfLds, SUB = kPotrfSub, NSUB = kPotrfBlock / SUB;
   double* S = psm;
   double* X = psm + kPotrfBlock * LDS;
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-    const int i = e / nb, j = e % nb;
-    S[i * LDS + j] = j <= i ? w[(int64_t)i * ld + j] : 0.0;
-  }
-  __syncthreads();
-  const bool ok = chol_in_smem(S, LDS, nb);
-  if (!ok) {
-    if (threadIdx.x == 0) atomicExch(notpd, 1);
-    return;
-  }
-  // column c of L11^-1: X[i][c] = -(sum_{c<=q<i} L[i][q] X[q][c]) / L[i][i], X[c][c] = 1 / L[c][c]
-  const int c = threadIdx.x;
-  if (c < kPotrfBlock) {
-    for (int i = 0; i < kPotrfBlock; ++i) {
-      double v = 0.0;
-      if (c < nb && i < nb && i >= c) {
-        double s = i == c ? 1.0 : 0.0;
-        for (int q = c; q < i; ++q) s = fma(-S[i * LDS + q], X[q * LDS + c], s);
-        v = s / S[i * LDS + i];
-      }
-      X[i * LDS + c] = v;
-    }
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-    const int i = e / nb, j = e % nb;
-    if (j <= i) w[(int64_t)i * ld + j] = S[i * LDS + j];
-  }
-  for (int e = threadIdx.x; e < kPotrfBlock * kPotrfBlock; e += blockDim.x) {
+  __shared__ double col[2][kPotrfBlock];
+  __shared__ int bad;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, q = lane & 3;
+  griddep_launch_dependents();
+  griddep_wait();  // the kernel before this one in the stream has completed
+  if (t == 0) bad = 0;
+#pragma unroll
+  for (int e = t; e < kPotrfBlock * kPotrfBlock; e += kPotrfThreads) {
     const int i = e / kPotrfBlock, j = e % kPotrfBlock;
-    linv[e] = X[i * LDS + j];
+    S[i * LDS + j] = i < nb ? (j <= i ? w[(int64_t)i * ld + j] : 0.0) : (i == j ? 1.0 : 0.0);
+    X[i * LDS + j] = 0.0;
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int c0 = 0; c0 < kPotrfBlock; c0 += SUB) {
+    if (t < kPotrfBlock) {
+      double p[SUB];
+#pragma unroll
+      for (int i = 0; i < SUB; ++i) p[i] = S[t * LDS + c0 + i];
+      bool ok = true;
+#pragma unroll
+      for (int i = 0; i < SUB; ++i) {
+        double* cb = col[i & 1];
+        cb[t] = p[i];
+        asm volatile("bar.sync 1, 64;" ::: "memory");
+        const double d0 = cb[c0 + i];
+        ok = ok && d0 > 0.0;
+        // a positive d0 has a normal square root: rustymath's divide multiplies by its reciprocal
+        const double d = sqrt(d0), r = 1.0 / d;
+        const double l = p[i] * r;
+        p[i] = t == c0 + i ? d : l;
+#pragma unroll
+        for (int j = i + 1; j < SUB; ++j) p[j] = fma(l, -(cb[c0 + j] * r), p[j]);
+      }
+      if (t >= c0) {
+#pragma unroll
+        for (int i = 0; i < SUB; ++i) S[t * LDS + c0 + i] = c0 + i <= t ? p[i] : 0.0;
+      }
+      if (!ok) bad = 1;
+    }
+    __syncthreads();
+    if (bad) {
+      if (t == 0) atomicExch(notpd, 1);
+      return;
+    }
+    // the later columns lose the 16: m16 x n8 tiles of the lower triangle
+    const int c1 = c0 + SUB, mt = (kPotrfBlock - c1) / 16;
+    for (int e = warp; e < mt * mt * 2; e += kPotrfThreads / 32) {
+      const int m0 = c1 + e / (2 * mt) * 16, n0 = c1 + e % (2 * mt) * 8;
+      if (n0 > m0 + 15) continue;
+      double* xa = S + (m0 + g) * LDS + n0 + 2 * q;
+      double* xb = xa + 8 * LDS;
+      double d[4] = {xa[0], xa[1], xb[0], xb[1]};
+#pragma unroll
+      for (int k = 0; k < SUB; k += 8) {
+        const double* a0 = S + (m0 + g) * LDS + c0 + k + q;
+        const double a[4] = {-a0[0], -a0[8 * LDS], -a0[4], -a0[8 * LDS + 4]};
+        const double* b0 = S + (n0 + g) * LDS + c0 + k + q;
+        potrf_mma(d, a, b0[0], b0[4]);
+      }
+      xa[0] = d[0], xa[1] = d[1], xb[0] = d[2], xb[1] = d[3];
+    }
+    __syncthreads();
+  }
+  // L back, and the diagonal blocks' inverses: x_i = (delta - sum) / l_ii, a lane per column
+  for (int e = t; e < kPotrfBlock * kPotrfBlock; e += kPotrfThreads) {
+    const int i = e / kPotrfBlock, j = e % kPotrfBlock;
+    if (i < nb && j <= i) w[(int64_t)i * ld + j] = S[i * LDS + j];
+  }
+  if (warp < NSUB && lane < SUB) {
+    const double* D = S + warp * SUB * LDS + warp * SUB;
+    double x[SUB];
+#pragma unroll
+    for (int i = 0; i < SUB; ++i) x[i] = i == lane ? 1.0 : 0.0;
+#pragma unroll
+    for (int i = 0; i < SUB; ++i) {
+      x[i] = x[i] / D[i * LDS + i];
+#pragma unroll
+      for (int r = i + 1; r < SUB; ++r) x[r] = fma(-D[r * LDS + i], x[i], x[r]);
+    }
+#pragma unroll
+    for (int i = 0; i < SUB; ++i) X[(warp * SUB + i) * LDS + warp * SUB + lane] = x[i];
+  }
+  __syncthreads();
+  // X_ba = -D_b^-1 sum_{a <= c < b} L_bc X_ca, by the distance b - a; a warp per 16 x 8 half
+  for (int dist = 1; dist < NSUB; ++dist) {
+    const int a = warp >> 1, b = a + dist, n0 = SUB * a + 8 * (warp & 1);
+    const bool mine = b < NSUB;
+    double* xa = X + (SUB * b + g) * LDS + n0 + 2 * q;
+    double* xb = xa + 8 * LDS;
+    if (mine) {
+      double d[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int k = SUB * a; k < SUB * b; k += 8) {
+        const double* a0 = S + (SUB * b + g) * LDS + k + q;
+        const double av[4] = {-a0[0], -a0[8 * LDS], -a0[4], -a0[8 * LDS + 4]};
+        const double* b0 = X + (k + q) * LDS + n0 + g;
+        potrf_mma(d, av, b0[0], b0[4 * LDS]);
+      }
+      xa[0] = d[0], xa[1] = d[1], xb[0] = d[2], xb[1] = d[3];
+    }
+    __syncwarp();  // a warp reads only its own columns of this block row
+    if (mine) {
+      double d[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int k = 0; k < SUB; k += 8) {
+        const double* a0 = X + (SUB * b + g) * LDS + SUB * b + k + q;
+        const double av[4] = {a0[0], a0[8 * LDS], a0[4], a0[8 * LDS + 4]};
+        const double* b0 = X + (SUB * b + k + q) * LDS + n0 + g;
+        potrf_mma(d, av, b0[0], b0[4 * LDS]);
+      }
+      __syncwarp();
+      xa[0] = d[0], xa[1] = d[1], xb[0] = d[2], xb[1] = d[3];
+    }
+    __syncthreads();
+  }
+  for (int e = t; e < kPotrfBlock * kPotrfBlock; e += kPotrfThreads) {
+    const int i = e / kPotrfBlock, j = e % kPotrfBlock;
+    linv[e] = i < nb && j < nb ? X[i * LDS + j] : 0.0;
   }
 }
 
@@ -142,8 +248,7 @@ __global__ void __launch_bounds__(kPotrfThreads) chol_small_kernel(const double*
 size_t potrf_f64_scratch_bytes(int64_t n) {
   const int64_t ld = round_up(std::max<int64_t>(n, 1), 32);
   return ((size_t)n * ld * 8 + 255) / 256 * 256                    // W
-         + (size_t)kPotrfBlock * kPotrfBlock * 8                   // L11^-1
-         + ((size_t)n * kPotrfBlock * 8 + 255) / 256 * 256 + 256;  // L21 before it goes back, the flag
+         + (size_t)kPotrfBlock * kPotrfBlock * 8 + 256;            // L11^-1, the flag
 }
 
 int potrf_f64(const double* a, int64_t n, double* l, void* scratch, int* notpd_host, unsigned* status,
@@ -153,29 +258,26 @@ int potrf_f64(const double* a, int64_t n, double* l, void* scratch, int* notpd_h
   char* base = static_cast<char*>(scratch);
   double* w = reinterpret_cast<double*>(base);
   double* linv = reinterpret_cast<double*>(base + ((size_t)n * ld * 8 + 255) / 256 * 256);
-  double* t = linv + kPotrfBlock * kPotrfBlock;
-  int* flag = reinterpret_cast<int*>(reinterpret_cast<char*>(t) + ((size_t)n * kPotrfBlock * 8 + 255) / 256 * 256);
+  int* flag = reinterpret_cast<int*>(linv + kPotrfBlock * kPotrfBlock);
   const int blocks = (int)std::min<int64_t>((n * ld + 255) / 256, 8 * device_sm_count());
   RM_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), stream));
   chol_load_kernel<<<blocks, 256, 0, stream>>>(a, n, w, ld);
   RM_LAUNCHED();
-  const size_t smem = (size_t)2 * kPotrfBlock * (kPotrfBlock + 1) * sizeof(double);
+  const size_t smem = (size_t)2 * kPotrfBlock * kPotrfLds * sizeof(double);
   RM_TRY(smem_attribute(potrf_diag_kernel, smem));
   for (int64_t k0 = 0; k0 < n; k0 += kPotrfBlock) {
     const int nb = (int)std::min<int64_t>(kPotrfBlock, n - k0);
     const int64_t rest = n - k0 - nb;
     double* a11 = w + k0 * ld + k0;
-    potrf_diag_kernel<<<1, kPotrfThreads, smem, stream>>>(a11, ld, nb, linv, flag);
-    RM_LAUNCHED();
+    RM_CUDA_TRY(launch_dependent(potrf_diag_kernel, dim3(1), dim3(kPotrfThreads), smem, stream, a11, ld, nb, linv, flag));
+    note_launch();
     if (rest == 0) break;
     double* a21 = a11 + (int64_t)nb * ld;
-    // L21 = A21 L11^-T into t, then back into W
-    RM_TRY(dgemm_device(false, true, rest, nb, nb, 1.0, a21, ld, linv, kPotrfBlock, 0.0, t, kPotrfBlock, status,
-                        stream));
-    RM_CUDA_TRY(cudaMemcpy2DAsync(a21, ld * 8, t, kPotrfBlock * 8, (size_t)nb * 8, rest, cudaMemcpyDeviceToDevice,
-                                  stream));
-    // A22 -= L21 L21^T
-    RM_TRY(dgemm_device(false, true, rest, rest, nb, -1.0, a21, ld, a21, ld, 1.0, a21 + nb, ld, status, stream));
+    // L21 = A21 L11^-T in place: nb <= 64 columns are one tile wide, so the CTA that stores a row is
+    // the only one that reads it, and has read it by then
+    RM_TRY(dgemm_device(false, true, rest, nb, nb, 1.0, a21, ld, linv, kPotrfBlock, 0.0, a21, ld, status, stream));
+    // A22 -= L21 L21^T, the tiles of the lower triangle
+    RM_TRY(dgemm_lower_device(rest, nb, -1.0, a21, ld, a21, ld, 1.0, a21 + nb, ld, status, stream));
   }
   if (notpd_host) RM_CUDA_TRY(cudaMemcpyAsync(notpd_host, flag, sizeof(int), cudaMemcpyDeviceToHost, stream));
   chol_store_kernel<<<(int)std::min<int64_t>((n * n + 255) / 256, 8 * device_sm_count()), 256, 0, stream>>>(w, ld, n,
