@@ -12,6 +12,13 @@ namespace rm {
 // kItemF64 when the precision tuner gave its size bucket float64 factors (no refinement).
 constexpr int kItemF64 = 1 << 8;
 
+constexpr int kBatchMaxK = 8;  // right-hand sides of a system
+
+// result flags per system
+constexpr int FLAG_FELL_BACK = 1;
+constexpr int FLAG_NOT_REGULAR = 2;
+constexpr int FLAG_NO_CONVERGENCE = 4;
+
 struct BatchArgs {
   int first, last;  // items [first, last) of the processing order
   const int* sys;   // item -> system

@@ -21,14 +21,9 @@ constexpr int NMAX = RM_BT_NMAX;  // rows of a system: a thread per row
 static_assert(NMAX == MAX_N, "the build's size class");
 constexpr int THREADS = NMAX;
 constexpr int WARPS = THREADS / 32;
-constexpr int KMAX = 8;    // right-hand sides of a system
+constexpr int KMAX = kBatchMaxK;
 constexpr int SLOT_BYTES = 144;
 constexpr int UBT_BYTES = NMAX * 144;  // U12 transposed (NMAX rows of 144 bytes), or row segments
-
-// result flags per system
-constexpr int FLAG_FELL_BACK = 1;
-constexpr int FLAG_NOT_REGULAR = 2;
-constexpr int FLAG_NO_CONVERGENCE = 4;
 
 struct Smem {
   alignas(16) unsigned char slot[2][WARPS][SLOT_BYTES];  // posts: NB items, then key (T), row
