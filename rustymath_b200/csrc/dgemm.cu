@@ -37,6 +37,7 @@ struct DgemmCfg {
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 2 * STAGES * 8;
   static constexpr int MI = WM / 16, NJ = WN / 8;
+  static constexpr bool PIPE = MI * NJ <= 2;  // few products per step, few warps: fetch a step ahead
   static_assert(BM % 16 == 0 && BN % 16 == 0 && WM % 16 == 0 && WN % 16 == 0, "tile shape");
   static_assert(BM <= 256 && BN <= 256, "TMA box extent");
 };
@@ -129,43 +130,99 @@ __global__ void __launch_bounds__(C::THREADS, 1)
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.0;
 
-  bool ok = true;
-  for (int kt = 0; kt < ktiles; ++kt) {
-    if (threadIdx.x == 0 && producing && issued < ktiles) issue(issued++);
-    const int s = kt % C::STAGES;
-    if (!mbar_wait(&full[s], (kt / C::STAGES) & 1u, status)) { ok = false; break; }
-    const uint8_t* sa = smem + s * C::STAGE_BYTES;
+  // The fragments of 8 k's. k offsets kk and kk + 4 change the swizzled chunk by XOR, so they are
+  // recomputed per k.
+  auto load_frags = [&](int st, int kk, double (&af)[C::MI][4], double (&bf)[C::NJ][2]) {
+    const uint8_t* sa = smem + st * C::STAGE_BYTES;
     const uint8_t* sb = sa + C::A_BYTES;
 #pragma unroll
-    for (int kk = 0; kk < C::BK; kk += 8) {
-      double af[C::MI][4], bf[C::NJ][2];
-#pragma unroll
-      for (int i = 0; i < C::MI; ++i) {
-        // k offsets kk and kk+4 change the swizzled chunk by XOR, so recompute per k.
-        const uint32_t r0 = arow(i, g), r1 = arow(i, g + 8);
-        af[i][0] = *reinterpret_cast<const double*>(sa + tile_off<!C::TA>(r0, kk + t));
-        af[i][1] = *reinterpret_cast<const double*>(sa + tile_off<!C::TA>(r1, kk + t));
-        af[i][2] = *reinterpret_cast<const double*>(sa + tile_off<!C::TA>(r0, kk + t + 4));
-        af[i][3] = *reinterpret_cast<const double*>(sa + tile_off<!C::TA>(r1, kk + t + 4));
-      }
-#pragma unroll
-      for (int j = 0; j < C::NJ; ++j) {
-        const uint32_t q = bcol(j, g);
-        bf[j][0] = *reinterpret_cast<const double*>(sb + tile_off<C::TB>(q, kk + t));
-        bf[j][1] = *reinterpret_cast<const double*>(sb + tile_off<C::TB>(q, kk + t + 4));
-      }
-#pragma unroll
-      for (int i = 0; i < C::MI; ++i)
-#pragma unroll
-        for (int j = 0; j < C::NJ; ++j)
-          asm volatile(
-              "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-              "{%0,%1,%2,%3};"
-              : "+d"(acc[i][j][0]), "+d"(acc[i][j][1]), "+d"(acc[i][j][2]), "+d"(acc[i][j][3])
-              : "d"(af[i][0]), "d"(af[i][1]), "d"(af[i][2]), "d"(af[i][3]), "d"(bf[j][0]), "d"(bf[j][1]));
+    for (int i = 0; i < C::MI; ++i) {
+      const uint32_t r0 = arow(i, g), r1 = arow(i, g + 8);
+      af[i][0] = *reinterpret_cast<const double*>(sa + tile_off<!C::TA>(r0, kk + t));
+      af[i][1] = *reinterpret_cast<const double*>(sa + tile_off<!C::TA>(r1, kk + t));
+      af[i][2] = *reinterpret_cast<const double*>(sa + tile_off<!C::TA>(r0, kk + t + 4));
+      af[i][3] = *reinterpret_cast<const double*>(sa + tile_off<!C::TA>(r1, kk + t + 4));
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[s]);
+#pragma unroll
+    for (int j = 0; j < C::NJ; ++j) {
+      const uint32_t q = bcol(j, g);
+      bf[j][0] = *reinterpret_cast<const double*>(sb + tile_off<C::TB>(q, kk + t));
+      bf[j][1] = *reinterpret_cast<const double*>(sb + tile_off<C::TB>(q, kk + t + 4));
+    }
+  };
+  auto multiply = [&](const double (&af)[C::MI][4], const double (&bf)[C::NJ][2]) {
+#pragma unroll
+    for (int i = 0; i < C::MI; ++i)
+#pragma unroll
+      for (int j = 0; j < C::NJ; ++j)
+        asm volatile(
+            "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+            "{%0,%1,%2,%3};"
+            : "+d"(acc[i][j][0]), "+d"(acc[i][j][1]), "+d"(acc[i][j][2]), "+d"(acc[i][j][3])
+            : "d"(af[i][0]), "d"(af[i][1]), "d"(af[i][2]), "d"(af[i][3]), "d"(bf[j][0]), "d"(bf[j][1]));
+  };
+
+  bool ok = true;
+  if constexpr (C::PIPE) {
+    // few warps per SM: the next 8 k's fragments are loaded before this step's products, so that
+    // neither the shared loads' latency nor a stage's barrier stands between products
+    double af[2][C::MI][4], bf[2][C::NJ][2];
+    ok = mbar_wait(&full[0], 0u, status);
+    if (ok) load_frags(0, 0, af[0], bf[0]);
+    for (int kt = 0; ok && kt < ktiles; ++kt) {
+      if (threadIdx.x == 0 && producing && issued < ktiles) issue(issued++);
+      const int s = kt % C::STAGES;
+      load_frags(s, 8, af[1], bf[1]);
+      multiply(af[0], bf[0]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[s]);  // the stage has been read
+      if (kt + 1 < ktiles) {
+        const int s1 = (kt + 1) % C::STAGES;
+        ok = mbar_wait(&full[s1], ((kt + 1) / C::STAGES) & 1u, status);
+        if (ok) load_frags(s1, 0, af[0], bf[0]);
+      }
+      multiply(af[1], bf[1]);
+    }
+  } else {
+    for (int kt = 0; kt < ktiles; ++kt) {
+      if (threadIdx.x == 0 && producing && issued < ktiles) issue(issued++);
+      const int s = kt % C::STAGES;
+      if (!mbar_wait(&full[s], (kt / C::STAGES) & 1u, status)) {
+        ok = false;
+        break;
+      }
+      const uint8_t* sa = smem + s * C::STAGE_BYTES;
+      const uint8_t* sb = sa + C::A_BYTES;
+#pragma unroll
+      for (int kk = 0; kk < C::BK; kk += 8) {
+        double af[C::MI][4], bf[C::NJ][2];
+#pragma unroll
+        for (int i = 0; i < C::MI; ++i) {
+          const uint32_t r0 = arow(i, g), r1 = arow(i, g + 8);
+          af[i][0] = *reinterpret_cast<const double*>(sa + tile_off<!C::TA>(r0, kk + t));
+          af[i][1] = *reinterpret_cast<const double*>(sa + tile_off<!C::TA>(r1, kk + t));
+          af[i][2] = *reinterpret_cast<const double*>(sa + tile_off<!C::TA>(r0, kk + t + 4));
+          af[i][3] = *reinterpret_cast<const double*>(sa + tile_off<!C::TA>(r1, kk + t + 4));
+        }
+#pragma unroll
+        for (int j = 0; j < C::NJ; ++j) {
+          const uint32_t q = bcol(j, g);
+          bf[j][0] = *reinterpret_cast<const double*>(sb + tile_off<C::TB>(q, kk + t));
+          bf[j][1] = *reinterpret_cast<const double*>(sb + tile_off<C::TB>(q, kk + t + 4));
+        }
+#pragma unroll
+        for (int i = 0; i < C::MI; ++i)
+#pragma unroll
+          for (int j = 0; j < C::NJ; ++j)
+            asm volatile(
+                "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+                "{%0,%1,%2,%3};"
+                : "+d"(acc[i][j][0]), "+d"(acc[i][j][1]), "+d"(acc[i][j][2]), "+d"(acc[i][j][3])
+                : "d"(af[i][0]), "d"(af[i][1]), "d"(af[i][2]), "d"(af[i][3]), "d"(bf[j][0]), "d"(bf[j][1]));
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[s]);
+    }
   }
   if (!ok) {
     // leave no copy in flight behind: wait (bounded) for every issued stage's bytes
@@ -433,16 +490,48 @@ static int launch_cfg(const double* a, int64_t lda, const double* b, int64_t ldb
   return RM_OK;
 }
 
+// The tile by the number of tiles: a launch lasts as long as its fullest SM does, so the tile is the
+// smallest whose tiles come to at most two or three per SM, and the stages are as many as leave room
+// for just that many CTAs (deeper stages hide more of the operands' latency, and the CTAs spread
+// evenly). Measured (us, one 64 x 64 tile of four warps before): 512^3 37 -> 18 with 32 x 32 tiles
+// at two per SM, 12 stages (27 with 6 stages and room for four); 640^3 72 -> 26 at three per SM;
+// 768^3 88 -> 37 with 64 x 32; 1024^3 128 -> 79 and 2135 x 3926 x 462 463 -> 294 with 64 x 64 at
+// two per SM (6 stages) in a stream of products, alone 90 and 320 either way; 1200^3 161 -> 144 at
+// three per SM (4 stages). From 148 tiles of 128 x 128 on, those.
+// whole_rows: the tile must span all n <= 128 columns (C may then be A: a CTA has read its rows'
+// items before it stores them).
 template <bool TA, bool TB>
 static int launch_t(const double* a, int64_t lda, const double* b, int64_t ldb, double* c, int64_t ldc, int m, int n,
-                    int k, double alpha, double beta, unsigned* status, cudaStream_t stream, bool wide) {
-  const int64_t big_tiles = ((int64_t)(m + 127) / 128) * ((n + 127) / 128);
-  if (wide || big_tiles >= device_sm_count()) {
-    using Big = DgemmCfg<128, 128, 64, 32, 4, TA, TB>;
-    return launch_cfg<Big>(a, lda, b, ldb, c, ldc, m, n, k, alpha, beta, status, stream);
+                    int k, double alpha, double beta, unsigned* status, cudaStream_t stream, bool whole_rows,
+                    bool lower = false) {
+  const int64_t sms = device_sm_count();
+  auto tiles = [&](int bm, int bn) {
+    const int64_t t = (int64_t)((m + bm - 1) / bm) * ((n + bn - 1) / bn);
+    return lower ? (t + 1) / 2 : t;
+  };
+  using Mid = DgemmCfg<64, 64, 32, 32, 6, TA, TB>;
+  using Big = DgemmCfg<128, 128, 64, 32, 4, TA, TB>;
+  if (whole_rows) {
+    if (n > Big::BN) return RM_BAD_ARG;
+    if (n <= Mid::BN) return launch_cfg<Mid>(a, lda, b, ldb, c, ldc, m, n, k, alpha, beta, status, stream, lower);
+    return launch_cfg<Big>(a, lda, b, ldb, c, ldc, m, n, k, alpha, beta, status, stream, lower);
   }
-  using Small = DgemmCfg<64, 64, 32, 32, 4, TA, TB>;
-  return launch_cfg<Small>(a, lda, b, ldb, c, ldc, m, n, k, alpha, beta, status, stream);
+  if (tiles(128, 128) >= sms)
+    return launch_cfg<Big>(a, lda, b, ldb, c, ldc, m, n, k, alpha, beta, status, stream, lower);
+  if (tiles(32, 32) <= 2 * sms)
+    return launch_cfg<DgemmCfg<32, 32, 16, 16, 12, TA, TB>>(a, lda, b, ldb, c, ldc, m, n, k, alpha, beta, status, stream,
+                                                            lower);
+  if (tiles(32, 32) <= 3 * sms)
+    return launch_cfg<DgemmCfg<32, 32, 16, 16, 8, TA, TB>>(a, lda, b, ldb, c, ldc, m, n, k, alpha, beta, status, stream,
+                                                           lower);
+  if (tiles(64, 32) <= 2 * sms)
+    return launch_cfg<DgemmCfg<64, 32, 16, 16, 8, TA, TB>>(a, lda, b, ldb, c, ldc, m, n, k, alpha, beta, status, stream,
+                                                           lower);
+  const int64_t t64 = tiles(64, 64);
+  if (t64 > 2 * sms && t64 <= 3 * sms)
+    return launch_cfg<DgemmCfg<64, 64, 32, 32, 4, TA, TB>>(a, lda, b, ldb, c, ldc, m, n, k, alpha, beta, status, stream,
+                                                           lower);
+  return launch_cfg<Mid>(a, lda, b, ldb, c, ldc, m, n, k, alpha, beta, status, stream, lower);
 }
 
 int dgemm_device(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha, const double* a, int64_t lda,
@@ -463,12 +552,7 @@ int dgemm_lower_device(int64_t n, int64_t k, double alpha, const double* a, int6
                        double beta, double* c, int64_t ldc, unsigned* status, cudaStream_t stream) {
   if (n == 0) return RM_OK;
   if (n > INT32_MAX || k < 1 || k > INT32_MAX) return RM_BAD_ARG;
-  const int64_t t = (n + 127) / 128, big_tiles = t * (t + 1) / 2;
-  if (big_tiles >= device_sm_count())
-    return launch_cfg<DgemmCfg<128, 128, 64, 32, 4, false, true>>(a, lda, b, ldb, c, ldc, (int)n, (int)n, (int)k, alpha,
-                                                                  beta, status, stream, true);
-  return launch_cfg<DgemmCfg<64, 64, 32, 32, 4, false, true>>(a, lda, b, ldb, c, ldc, (int)n, (int)n, (int)k, alpha, beta,
-                                                              status, stream, true);
+  return launch_t<false, true>(a, lda, b, ldb, c, ldc, (int)n, (int)n, (int)k, alpha, beta, status, stream, false, true);
 }
 
 // C = beta*C (beta == 0 writes zeros), the reference's `scale` (linalg.rs:1000-1008).

@@ -273,9 +273,10 @@ int potrf_f64(const double* a, int64_t n, double* l, void* scratch, int* notpd_h
     note_launch();
     if (rest == 0) break;
     double* a21 = a11 + (int64_t)nb * ld;
-    // L21 = A21 L11^-T in place: nb <= 64 columns are one tile wide, so the CTA that stores a row is
-    // the only one that reads it, and has read it by then
-    RM_TRY(dgemm_device(false, true, rest, nb, nb, 1.0, a21, ld, linv, kPotrfBlock, 0.0, a21, ld, status, stream));
+    // L21 = A21 L11^-T in place, a tile as wide as the block: the CTA that stores a row is the only
+    // one that reads it, and has read it by then
+    RM_TRY(dgemm_device(false, true, rest, nb, nb, 1.0, a21, ld, linv, kPotrfBlock, 0.0, a21, ld, status, stream,
+                        /*whole_rows=*/true));
     // A22 -= L21 L21^T, the tiles of the lower triangle
     RM_TRY(dgemm_lower_device(rest, nb, -1.0, a21, ld, a21, ld, 1.0, a21 + nb, ld, status, stream));
   }

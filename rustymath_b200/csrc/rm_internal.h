@@ -9,11 +9,11 @@ namespace rm {
 
 // ---------------------------------------------------------------- GEMM (dgemm.cu)
 // C = alpha*op(A)*op(B) + beta*C, row-major; a, b 16-byte aligned with even lda, ldb.
-// `force_wide_m` picks the 128-row tile whatever the size, which makes a product whose
-// m <= 128 read each column block of B in one CTA (so B may alias C).
+// `whole_rows` picks a tile that spans all n <= 128 columns, so that C may be A (a CTA stores rows that
+// only it has read).
 int dgemm_device(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha, const double* a, int64_t lda,
                  const double* b, int64_t ldb, double beta, double* c, int64_t ldc, unsigned* status,
-                 cudaStream_t stream, bool force_wide_m = false);
+                 cudaStream_t stream, bool whole_rows = false);
 int scale_device(double* c, int64_t ldc, int64_t m, int64_t n, double beta, cudaStream_t stream);
 // C = alpha op(A) op(B) + beta C for m == 1 or n == 1 (k >= 1, alpha != 0): streams over the
 // matrix operand instead of DMMA tiles (gemv.cu)

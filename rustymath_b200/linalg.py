@@ -568,11 +568,7 @@ def matmul_ozaki(a, b, slices=8):
 def _gemm(a, b, device):
     m, k = a.shape
     n = b.shape[1]
-    c = _empty((m, n), a, device)
-    if device and m * n:
-        c.zero_()
-    elif m * n:
-        c.fill(0.0)
+    c = _empty((m, n), a, device)  # beta is 0: every item is written
     if m and n:
         lib = _lib.load()
         if device:
