@@ -34,6 +34,8 @@
 // that kernel's end; it reads nothing of it before griddepcontrol.wait).
 #include <climits>
 
+#include <cfloat>
+
 #include "rm_internal.h"
 
 namespace rm {
@@ -42,7 +44,7 @@ constexpr int kLppCols = 128;  // panel width (the trailing update's rank)
 constexpr int kLppRows = 256;  // rows a panel's pivots are chosen among
 constexpr int kLppLeaf = 16;
 constexpr int kLppThreads = 256;  // a thread per row
-constexpr int kLppStride = kLppCols + 1;
+constexpr int kLppStride = kLppCols + 4;  // 16-byte rows, an odd number of 16-byte pieces apart
 
 __device__ __forceinline__ void warp_argmax_f32(float& v, int& i) {
 #pragma unroll
@@ -82,6 +84,20 @@ __device__ __forceinline__ unsigned pivot_key(float v) {
   return a != a ? 1u : __float_as_uint(a) + 2u;
 }
 
+// 1 / a from the hardware's approximation and one Newton step x += x (1 - a x), within an ulp. The
+// correctly rounded sequence branches and takes ~130 cycles, on the path of every column; this runs
+// beside the reduction. Where the step is not finite the approximation stands (0 for an infinity).
+__device__ __forceinline__ float lpp_rcp(float a) {
+  float x;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(x) : "f"(a));
+  const float y = fmaf(x, fmaf(-a, x, 1.0f), x);
+  return fabsf(y) <= FLT_MAX ? y : x;
+}
+
+// Where U12's column j of a leaf is staged: a tile's lanes read columns 4 q + i together, so those
+// lie next to each other.
+__device__ __forceinline__ int lpp_ub_at(int j) { return (j & ~31) | ((j & 3) << 3) | ((j >> 2) & 7); }
+
 // Factors the T x nb panel A[j0.., j0..] (T <= 256, nb <= 128) with partial pivoting among
 // its T rows. Thread r owns row r. Pivoting is implicit: rows stay where they are and a row
 // chosen as a pivot leaves the candidates; the panel is written back in pivot order at the
@@ -115,16 +131,9 @@ __global__ void __launch_bounds__(kLppThreads, 1) lpp_panel_kernel(float* __rest
   griddep_launch_dependents();
   griddep_wait();  // the update of these columns has completed
   if (nb == kLppCols) {
-    // asynchronous 4-byte copies, every one of a thread's in flight at once: a warp per row,
-    // lane l the row's floats 4l..4l+3 (each warp reads 512 contiguous bytes per row), in an
-    // order rotated by l / 8 so that the shared-memory writes of a warp hit 32 distinct banks
-    const int rot = lane >> 3;
-    for (int rr = warp; rr < T; rr += kLppThreads / 32)
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const int c = 4 * lane + ((t + rot) & 3);
-        cp_async4(&P[rr][c], blk + (int64_t)rr * lda + c);
-      }
+    // asynchronous 16-byte copies, every one of a thread's in flight at once: a warp per row (lda is a
+    // multiple of 32 and j0 of 128)
+    for (int rr = warp; rr < T; rr += kLppThreads / 32) cp_async16(&P[rr][4 * lane], blk + (int64_t)rr * lda + 4 * lane);
     cp_async_wait_all();
   } else {
     for (int e = tid; e < T * nb; e += kLppThreads) {
@@ -147,7 +156,7 @@ __global__ void __launch_bounds__(kLppThreads, 1) lpp_panel_kernel(float* __rest
       // the warp's candidate: the largest key (redux), the lowest lane holding it (ballot);
       // every lane's reciprocal is taken while the reduction runs, the winner posts its own
       const unsigned key = active ? pivot_key(p[c]) : 0u;
-      const float myrcp = __frcp_rn(p[c]);
+      const float myrcp = lpp_rcp(p[c]);
       const unsigned wmax = __reduce_max_sync(0xffffffffu, key);
       const int wl = __ffs(__ballot_sync(0xffffffffu, key == wmax)) - 1;
       if (lane == wl) {
@@ -223,24 +232,47 @@ __global__ void __launch_bounds__(kLppThreads, 1) lpp_panel_kernel(float* __rest
 #pragma unroll
       for (int c = 0; c < kLppLeaf; ++c) {
         P[piv_s[c0 + c]][rc0 + j] = u[c];
-        UbT[j][c] = u[c];
+        UbT[lpp_ub_at(j)][c] = u[c];
       }
     }
     __syncthreads();
-    // the rows still unchosen: later columns -= L(row, leaf) U12
-    if (active) {
-      for (int j = 0; j < rcols; ++j) {
-        float a0 = P[r][rc0 + j], a1 = 0.f, a2 = 0.f, a3 = 0.f;  // four chains
-        const float4* ub = reinterpret_cast<const float4*>(&UbT[j][0]);
+    // the rows still unchosen: later columns -= L(row, leaf) U12. A warp takes its own 32 rows, 32
+    // columns at a time: lane (rg, cq) rows rg, rg + 4, ... and columns 4 cq .. 4 cq + 3, so that three
+    // 16-byte shared loads serve 32 FMAs. (A row per thread reads U12's 16 items for each of its
+    // items: 16 wavefronts of the SM's one shared-memory pipe per 16 FMAs, half the panel's time.)
+    {
+      const unsigned live = __ballot_sync(0xffffffffu, active);
+      const int rg = lane >> 3, cq = lane & 7;
+      const float* rows = &P[32 * warp + rg][0];
+      for (int n0 = 0; live != 0u && n0 + 4 * cq < rcols; n0 += 32) {
+        float x[8][4];
 #pragma unroll
-        for (int q = 0; q < kLppLeaf / 4; ++q) {
-          const float4 u4 = ub[q];
-          a0 = fmaf(-p[4 * q], u4.x, a0);
-          a1 = fmaf(-p[4 * q + 1], u4.y, a1);
-          a2 = fmaf(-p[4 * q + 2], u4.z, a2);
-          a3 = fmaf(-p[4 * q + 3], u4.w, a3);
+        for (int i = 0; i < 8; ++i) {
+          const float4 v = *reinterpret_cast<const float4*>(rows + 4 * i * kLppStride + rc0 + n0 + 4 * cq);
+          x[i][0] = v.x, x[i][1] = v.y, x[i][2] = v.z, x[i][3] = v.w;
         }
-        P[r][rc0 + j] = (a0 + a1) + (a2 + a3);
+#pragma unroll
+        for (int k = 0; k < kLppLeaf; k += 4) {
+          float4 u[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) u[j] = *reinterpret_cast<const float4*>(&UbT[n0 + 8 * j + cq][k]);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float4 l = *reinterpret_cast<const float4*>(rows + 4 * i * kLppStride + c0 + k);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              x[i][j] = fmaf(-l.x, u[j].x, x[i][j]);
+              x[i][j] = fmaf(-l.y, u[j].y, x[i][j]);
+              x[i][j] = fmaf(-l.z, u[j].z, x[i][j]);
+              x[i][j] = fmaf(-l.w, u[j].w, x[i][j]);
+            }
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if ((live >> (rg + 4 * i)) & 1u)
+            *reinterpret_cast<float4*>(&P[32 * warp + rg + 4 * i][rc0 + n0 + 4 * cq]) =
+                make_float4(x[i][0], x[i][1], x[i][2], x[i][3]);
       }
     }
     __syncthreads();
