@@ -21,54 +21,6 @@ constexpr int kPreKC = 8;           // columns per chain of the scaled float32 s
 
 size_t diag_blocks_f64_bytes(int64_t n) { return diag_blocks_bytes_max(n); }
 
-// dinv[b][0] = inverse of the lower diagonal block b, dinv[b][1] = inverse of the upper
-// diagonal block b (row-major TB x TB; rows/columns past n are identity); dinv[b][2..3] are
-// the couplings that coupling_kernel fills in. A unit triangle
-// takes its diagonal as 1 without reading it. The triangles are those of the n x n matrix
-// T whose item (i, j) is w[i*ldw + j], or w[j*ldw + i] when COLMAJOR. Thread c solves for
-// column c of the inverse.
-template <typename T, bool COLMAJOR, int TB>
-__global__ void __launch_bounds__(TB) invert_diag_blocks_kernel(const T* __restrict__ w, int64_t ldw, int64_t n,
-                                                                T* __restrict__ dinv, bool lower_unit, bool upper_unit) {
-  extern __shared__ uint8_t smraw[];
-  T(*x)[TB + 1] = reinterpret_cast<T(*)[TB + 1]>(smraw);
-  T(*t)[TB + 1] = reinterpret_cast<T(*)[TB + 1]>(smraw + (size_t)TB * (TB + 1) * sizeof(T));
-  const int b = blockIdx.x, which = blockIdx.y;  // 0: L, 1: U
-  const int64_t r0 = (int64_t)b * TB;
-  const int rows = (int)(n - r0 < TB ? n - r0 : TB);
-  const T* blk = w + r0 * ldw + r0;
-  const int col = threadIdx.x;
-  // the block in shared memory first (read along its storage order, coalesced); past n, identity
-  for (int e = threadIdx.x; e < TB * TB; e += blockDim.x) {
-    const int s0 = e / TB, s1 = e % TB;  // s1 runs along the storage
-    const int i = COLMAJOR ? s1 : s0, j = COLMAJOR ? s0 : s1;
-    t[i][j] = (i >= rows || j >= rows) ? (i == j ? T(1) : T(0))
-                                       : (COLMAJOR ? blk[(int64_t)j * ldw + i] : blk[(int64_t)i * ldw + j]);
-  }
-  __syncthreads();
-  auto A = [&](int i, int j) -> T { return t[i][j]; };
-  if (which == 0) {
-    // lower: x_i = (delta_i,col - sum_{col<=k<i} L_ik x_k) / L_ii for i >= col
-    for (int i = 0; i < TB; ++i) {
-      T s = i == col ? T(1) : T(0);
-      if (i > col)
-        for (int k = col; k < i; ++k) s = fma(-A(i, k), x[k][col], s);
-      x[i][col] = i < col ? T(0) : (lower_unit ? s : s / A(i, i));
-    }
-  } else {
-    // upper: x_i = (delta_i,col - sum_{i<k<=col} U_ik x_k) / U_ii for i <= col
-    for (int i = TB - 1; i >= 0; --i) {
-      T s = i == col ? T(1) : T(0);
-      if (i < col)
-        for (int k = i + 1; k <= col; ++k) s = fma(-A(i, k), x[k][col], s);
-      x[i][col] = i > col ? T(0) : (upper_unit ? s : s / A(i, i));
-    }
-  }
-  __syncthreads();
-  T* out = dinv + ((int64_t)b * kDiagMats + which) * TB * TB;
-  for (int e = threadIdx.x; e < TB * TB; e += blockDim.x) out[e] = x[e / TB][e % TB];
-}
-
 // out (TB x TB, row-major, ld ldo) = dinv block dv (TB x TB row-major) times block (b, pb) of
 // the n x n matrix T (item (i, j) at w[i*ldw + j], or at w[j*ldw + i] when COLMAJOR; past n,
 // zero). 256 threads, each a (TB/16)^2 piece; smem holds both operands.
@@ -128,28 +80,161 @@ __global__ void __launch_bounds__(256) coupling_kernel(const T* __restrict__ w, 
 }
 
 
-template <typename T, bool COLMAJOR, int TB>
-static int launch_invert(const T* w, int64_t ldw, int64_t n, T* dinv, bool lower_unit, bool upper_unit,
-                         cudaStream_t stream) {
-  const size_t smem = (size_t)TB * (TB + 1) * sizeof(T);
-  RM_TRY(smem_attribute(invert_diag_blocks_kernel<T, COLMAJOR, TB>, 2 * smem));
-  RM_TRY(smem_attribute(coupling_kernel<T, COLMAJOR, TB>, 2 * smem));
-  dim3 grid((unsigned)((n + TB - 1) / TB), 2);
-  invert_diag_blocks_kernel<T, COLMAJOR, TB><<<grid, TB, 2 * smem, stream>>>(w, ldw, n, dinv, lower_unit,
-                                                                              upper_unit);
-  RM_LAUNCHED();
-  if (grid.x > 1) {
-    coupling_kernel<T, COLMAJOR, TB><<<grid, 256, 2 * smem, stream>>>(w, ldw, n, dinv);
-    RM_LAUNCHED();
+// The solves' table of a triangle pair: dinv[b][0] = inverse of the lower diagonal block b,
+// dinv[b][1] = inverse of the upper diagonal block b (row-major TB x TB; rows/columns past n are
+// identity); dinv[b][2..3] the couplings. A unit triangle takes its diagonal as 1 without reading
+// it. The triangles are those of the n x n matrix T whose item (i, j) is w[i*ldw + j], or
+// w[j*ldw + i] when COLMAJOR.
+//
+// The float64 table in one launch: a CTA per (64-row block b, triangle) forms the inverse D_b^-1 of its
+// diagonal block and its coupling D_b^-1 T[b, b -+ 1] (zero past n). An upper triangle is inverted as
+// the lower triangle of its transpose. The inverse is put together from its four 16 x 16 diagonal
+// blocks' inverses (a warp each, a lane per column) on DMMA, block by the distance from the
+// diagonal; the coupling is one 64 x 64 x 64 product on DMMA whose operand came in meanwhile. A
+// thread per column running down the whole block (64 dependent steps of up to 64 shared-memory
+// products), and a second launch for the couplings, took 54 + 15 us at n = 512.
+constexpr int kD64Lds = kTB64 + 4;  // fragment loads of either orientation hit 16 distinct 8-byte banks
+constexpr size_t kD64Smem = (size_t)3 * kTB64 * kD64Lds * sizeof(double);
+
+__device__ __forceinline__ void d64_mma(double (&d)[4], const double (&a)[4], double b0, double b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b0), "d"(b1));
+}
+
+template <bool COLMAJOR>
+__global__ void __launch_bounds__(256) diag64_kernel(const double* __restrict__ w, int64_t ldw, int64_t n,
+                                                     double* __restrict__ dinv, bool lower_unit, bool upper_unit) {
+  constexpr int TB = kTB64, LDS = kD64Lds, SUB = 16, NSUB = TB / SUB;
+  extern __shared__ __align__(16) double dsm64[];
+  double* S = dsm64;           // the triangle, lower
+  double* X = S + TB * LDS;    // its inverse
+  double* B = X + TB * LDS;    // the neighbouring block
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, q = lane & 3;
+  const int b = blockIdx.x, which = blockIdx.y, nblk = (int)gridDim.x;  // 0: L, 1: U
+  const int64_t r0 = (int64_t)b * TB;
+  const int rows = (int)(n - r0 < TB ? n - r0 : TB);
+  const int pb = which == 0 ? b - 1 : b + 1;
+  const bool couple = pb >= 0 && pb < nblk, unit = which == 0 ? lower_unit : upper_unit;
+  const int64_t c0 = (int64_t)pb * TB;
+  {
+    const double* blk = w + r0 * ldw + r0;
+    double v[TB * TB / 256], u[TB * TB / 256];
+#pragma unroll
+    for (int i = 0; i < TB * TB / 256; ++i) {
+      const int s0 = (t + 256 * i) / TB, s1 = (t + 256 * i) % TB;  // s1 runs along the storage
+      v[i] = s0 < rows && s1 < rows ? blk[s0 * ldw + s1] : (s0 == s1 ? 1.0 : 0.0);
+      // item (r0 + ., c0 + .) of the neighbour, along the storage too
+      const int64_t o0 = (COLMAJOR ? c0 : r0) + s0, o1 = (COLMAJOR ? r0 : c0) + s1;
+      u[i] = couple && o0 < n && o1 < n ? w[o0 * ldw + o1] : 0.0;
+    }
+#pragma unroll
+    for (int i = 0; i < TB * TB / 256; ++i) {
+      const int s0 = (t + 256 * i) / TB, s1 = (t + 256 * i) % TB;
+      const int ti = COLMAJOR ? s1 : s0, tj = COLMAJOR ? s0 : s1;
+      const int li = which == 0 ? ti : tj, lj = which == 0 ? tj : ti;  // its place in the lower form
+      S[li * LDS + lj] = lj > li ? 0.0 : (unit && li == lj ? 1.0 : v[i]);
+      B[ti * LDS + tj] = u[i];
+      X[s0 * LDS + s1] = 0.0;
+    }
   }
-  return RM_OK;
+  __syncthreads();
+  if (warp < NSUB && lane < SUB) {
+    const double* D = S + warp * SUB * LDS + warp * SUB;
+    double x[SUB];
+#pragma unroll
+    for (int i = 0; i < SUB; ++i) x[i] = i == lane ? 1.0 : 0.0;
+#pragma unroll
+    for (int i = 0; i < SUB; ++i) {
+      if (!unit && i >= lane) x[i] = x[i] / D[i * LDS + i];
+#pragma unroll
+      for (int r = i + 1; r < SUB; ++r) x[r] = fma(-D[r * LDS + i], x[i], x[r]);
+    }
+#pragma unroll
+    for (int i = 0; i < SUB; ++i) X[(warp * SUB + i) * LDS + warp * SUB + lane] = x[i];
+  }
+  __syncthreads();
+  // X_ba = -D_b^-1 sum_{a <= c < b} S_bc X_ca, by the distance b - a; a warp per 16 x 8 half
+  for (int dist = 1; dist < NSUB; ++dist) {
+    const int ca = warp >> 1, cb = ca + dist, n0 = SUB * ca + 8 * (warp & 1);
+    const bool mine = cb < NSUB;
+    double* xa = X + (SUB * cb + g) * LDS + n0 + 2 * q;
+    double* xb = xa + 8 * LDS;
+    if (mine) {
+      double d[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int k = SUB * ca; k < SUB * cb; k += 8) {
+        const double* a0 = S + (SUB * cb + g) * LDS + k + q;
+        const double av[4] = {-a0[0], -a0[8 * LDS], -a0[4], -a0[8 * LDS + 4]};
+        const double* b0 = X + (k + q) * LDS + n0 + g;
+        d64_mma(d, av, b0[0], b0[4 * LDS]);
+      }
+      xa[0] = d[0], xa[1] = d[1], xb[0] = d[2], xb[1] = d[3];
+    }
+    __syncwarp();  // a warp reads only its own columns of this block row
+    if (mine) {
+      double d[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int k = 0; k < SUB; k += 8) {
+        const double* a0 = X + (SUB * cb + g) * LDS + SUB * cb + k + q;
+        const double av[4] = {a0[0], a0[8 * LDS], a0[4], a0[8 * LDS + 4]};
+        const double* b0 = X + (SUB * cb + k + q) * LDS + n0 + g;
+        d64_mma(d, av, b0[0], b0[4 * LDS]);
+      }
+      __syncwarp();
+      xa[0] = d[0], xa[1] = d[1], xb[0] = d[2], xb[1] = d[3];
+    }
+    __syncthreads();
+  }
+  double* out = dinv + ((int64_t)b * kDiagMats + which) * TB * TB;
+  for (int e = t; e < TB * TB; e += 256) {
+    const int i = e / TB, j = e % TB;
+    out[e] = which == 0 ? X[i * LDS + j] : X[j * LDS + i];
+  }
+  if (!couple) return;
+  // the coupling: warp w rows 16 (w / 2) .., columns 32 (w % 2) ..
+  out = dinv + ((int64_t)b * kDiagMats + 2 + which) * TB * TB;
+  const int m0 = 16 * (warp >> 1), n0 = 32 * (warp & 1);
+  double d[4][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) d[j][0] = d[j][1] = d[j][2] = d[j][3] = 0.0;
+#pragma unroll 2
+  for (int k = 0; k < TB; k += 8) {
+    double av[4];
+    if (which == 0) {
+      const double* a0 = X + (m0 + g) * LDS + k + q;
+      av[0] = a0[0], av[1] = a0[8 * LDS], av[2] = a0[4], av[3] = a0[8 * LDS + 4];
+    } else {  // U^-1 = X^T
+      const double* a0 = X + (k + q) * LDS + m0 + g;
+      av[0] = a0[0], av[1] = a0[8], av[2] = a0[4 * LDS], av[3] = a0[4 * LDS + 8];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const double* b0 = B + (k + q) * LDS + n0 + 8 * j + g;
+      d64_mma(d[j], av, b0[0], b0[4 * LDS]);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int col = n0 + 8 * j + 2 * q;
+    *reinterpret_cast<double2*>(out + (m0 + g) * TB + col) = make_double2(d[j][0], d[j][1]);
+    *reinterpret_cast<double2*>(out + (m0 + g + 8) * TB + col) = make_double2(d[j][2], d[j][3]);
+  }
 }
 
 int invert_diag_blocks_f64(const double* w, int64_t ldw, bool colmajor, int64_t n, double* dinv, bool lower_unit,
                            bool upper_unit, cudaStream_t stream) {
   if (n == 0) return RM_OK;
-  if (colmajor) return launch_invert<double, true, kTB64>(w, ldw, n, dinv, lower_unit, upper_unit, stream);
-  return launch_invert<double, false, kTB64>(w, ldw, n, dinv, lower_unit, upper_unit, stream);
+  const dim3 grid((unsigned)((n + kTB64 - 1) / kTB64), 2);
+  if (colmajor) {
+    RM_TRY(smem_attribute(diag64_kernel<true>, kD64Smem));
+    diag64_kernel<true><<<grid, 256, kD64Smem, stream>>>(w, ldw, n, dinv, lower_unit, upper_unit);
+  } else {
+    RM_TRY(smem_attribute(diag64_kernel<false>, kD64Smem));
+    diag64_kernel<false><<<grid, 256, kD64Smem, stream>>>(w, ldw, n, dinv, lower_unit, upper_unit);
+  }
+  RM_LAUNCHED();
+  return RM_OK;
 }
 
 __device__ __forceinline__ int ld_acquire(const int* p) {
@@ -744,11 +829,6 @@ int trsm_f64(bool right, bool lower, bool trans, bool unit, int64_t m, int64_t n
 
 size_t diag_blocks_f32_bytes(int64_t n) {
   return (size_t)((n + kTB32 - 1) / kTB32) * kDiagMats * kTB32 * kTB32 * sizeof(float);
-}
-
-int invert_diag_blocks_f32(const float* w, int64_t ldw, int64_t n, float* dinv, cudaStream_t stream) {
-  if (n == 0) return RM_OK;
-  return launch_invert<float, false, kTB32>(w, ldw, n, dinv, true, false, stream);
 }
 
 int couplings_f32(const float* w, int64_t ldw, int64_t n, float* dinv, cudaStream_t stream) {
