@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "rm_internal.h"
+#include "small_solve.cuh"
 
 namespace rm {
 
@@ -113,6 +114,7 @@ struct alignas(16) CallResults {
   unsigned status;
   int32_t flag;
   double berr[2];
+  SmallSolveResults small;
 };
 
 static CallResults* call_results() {
@@ -298,7 +300,7 @@ static LuBuffers plan_lu(Arena& arena, int64_t n) {
   b.w = arena.add((size_t)n * b.ldw * sizeof(double));
   b.ipiv = arena.add((size_t)n * sizeof(int64_t));
   b.perm = arena.add((size_t)n * sizeof(int64_t));
-  b.amax = arena.add(sizeof(double));
+  b.amax = arena.add(kSmallSolveParts * sizeof(double));
   b.flag = arena.add(sizeof(int32_t));
   b.dinv = arena.add(diag_blocks_f64_bytes(n));
   b.getrf = arena.add(getrf_f64_scratch_bytes(n));
@@ -755,6 +757,22 @@ static int dsolve_plain(int64_t n, const double* d_a, const double* d_b, int64_t
   RM_TRY(scratch_alloc(&sc.base, ar.total, s));
   double* w = sc.at<double>(lb.w);
   PhaseTrace tr(s, "plain float64 solve");
+  if (!report) {
+    CallResults* h = call_results();
+    unsigned* dst = device_status();
+    int st = RM_OK;
+    if (h && dst && small_plain_solve_f64(d_a, w, lb.ldw, n, d_b, k, d_x, sc.at<int64_t>(lb.ipiv),
+                                          sc.at<int64_t>(lb.perm), sc.at<double>(lb.amax), dst, &h->small, s, &st)) {
+      RM_TRY(st);
+      RM_CUDA_TRY(cudaStreamSynchronize(s));
+      RM_TRY(status_from_word(h->small.status, dst, s));
+      if (!h->small.flag) {
+        set_last_message("a pivot is at most eps*n*max|a|; rustymath's solve takes least squares here");
+        return RM_NOT_REGULAR;
+      }
+      return RM_OK;
+    }
+  }
   RM_TRY(load_matrix_f64(d_a, n, w, lb.ldw, n, sc.at<double>(lb.amax), s));
   tr.mark("load");
   RM_TRY(getrf_f64(w, lb.ldw, n, sc.at<int64_t>(lb.ipiv), sc.at<int64_t>(lb.perm), sc.at<void>(lb.getrf),

@@ -31,6 +31,7 @@
 #include "rm_cluster.cuh"
 #include "rm_internal.h"
 #include "short_pivot.cuh"
+#include "small_solve.cuh"
 
 namespace rm {
 
@@ -278,12 +279,13 @@ __device__ __forceinline__ void cluster_lu_post(ClusterLuShared& sh, int slot, d
   }
 }
 
-// W (row-major, ldw) is factored in place: on return row i of W holds row i of the factors (the
+// The n x n row-major a (lda; it may be W) is factored into W (row-major, ldw): on return row i of W
+// holds row i of the factors (the
 // source row perm[i]); ipiv[j] is the position exchanged with j at step j. R rows per CTA, ld
 // the shared row stride (odd: a warp's column reads hit distinct banks).
 __global__ void __launch_bounds__(32 * (1 + kClusterLuMax / 32), 1)
-    cluster_lu_kernel(double* __restrict__ w, int64_t ldw, int n, int R, int ld, int64_t* __restrict__ ipiv,
-                      int64_t* __restrict__ perm) {
+    cluster_lu_kernel(const double* a, int64_t lda, double* w, int64_t ldw, int n, int R, int ld,
+                      int64_t* __restrict__ ipiv, int64_t* __restrict__ perm, double* amax) {
   extern __shared__ __align__(16) uint8_t smem[];
   ClusterLuShared& sh = *reinterpret_cast<ClusterLuShared*>(smem);
   double* S = reinterpret_cast<double*>(smem + sizeof(ClusterLuShared));
@@ -292,8 +294,24 @@ __global__ void __launch_bounds__(32 * (1 + kClusterLuMax / 32), 1)
   const int rank = (int)cluster_ctarank(), C = (int)cluster_nctarank();
   const int g0 = rank * R;
   const int rows = max(0, min(R, n - g0));
+  double top = 0.0;
   for (int i = warp; i < rows; i += nwarps)
-    for (int c = lane; c < n; c += 32) S[i * ld + c] = w[(int64_t)(g0 + i) * ldw + c];
+    for (int c = lane; c < n; c += 32) {
+      const double v = a[(int64_t)(g0 + i) * lda + c];
+      S[i * ld + c] = v;
+      if (fabs(v) > top) top = fabs(v);  // NaN never is
+    }
+  if (amax != nullptr) {
+    __shared__ double tops[1 + kClusterLuMax / 32];
+#pragma unroll
+    for (int off = 16; off; off >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, off));
+    if (lane == 0) tops[warp] = top;
+    __syncthreads();
+    if (t == 0) {
+      for (int v = 1; v < nwarps; ++v) top = fmax(top, tops[v]);
+      amax[rank] = top;
+    }
+  }
   const bool valid = lane < rows;
   int pos = valid ? g0 + lane : INT_MAX;
   double* myrow = S + (valid ? lane : 0) * ld;
@@ -410,7 +428,8 @@ __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
 template <bool COLMAJOR>
 __global__ void __launch_bounds__(kSmallSolveMax, 1)
     small_solve_kernel(const double* __restrict__ w, int64_t ldw, int n, const int64_t* __restrict__ perm,
-                       const double* b, int k, double* x, unsigned* status) {
+                       const double* b, int k, double* x, unsigned* status, const double* amax, int parts,
+                       SmallSolveResults* results) {
   extern __shared__ __align__(16) uint8_t smem[];
   double* buf = reinterpret_cast<double*>(smem);  // two staging buffers of kSsCols * kSsStride * ... doubles
   __shared__ double xs[2][kSmallSolveK];
@@ -494,6 +513,18 @@ __global__ void __launch_bounds__(kSmallSolveMax, 1)
 #pragma unroll
     for (int c = 0; c < kSmallSolveK; ++c)
       if (c < k) x[(int64_t)t * k + c] = v[c];
+  if (results != nullptr) {
+    // LuWork::regular (regular_kernel), and what the caller reads, straight into its host memory
+    double top = 0.0;
+    for (int i = 0; i < parts; ++i) top = fmax(top, amax[i]);
+    const bool bad = own && fabs(w[(int64_t)t * ldw + t]) <= 2.220446049250313e-16 * (double)n * top;
+    const int any = __syncthreads_or(bad ? 1 : 0);
+    if (t == 0) {
+      results->flag = any ? 0 : 1;
+      results->status = *status;
+      __threadfence_system();
+    }
+  }
 }
 
 // The plain solve takes this kernel up to n = 192: measured per solve (n = 8 / 32 / 64 / 128 / 192 / 256,
@@ -508,11 +539,11 @@ int small_solve_f64(const double* w, int64_t ldw, bool colmajor, int64_t n, cons
   if (colmajor) {
     RM_TRY(smem_attribute(small_solve_kernel<true>, (size_t)2 * kSsCols * kSmallSolveMax * sizeof(double)));
     small_solve_kernel<true><<<1, kSmallSolveMax, (size_t)2 * kSsCols * n * sizeof(double), stream>>>(
-        w, ldw, (int)n, perm, b, (int)k, x, status);
+        w, ldw, (int)n, perm, b, (int)k, x, status, nullptr, 0, nullptr);
   } else {
     RM_TRY(smem_attribute(small_solve_kernel<false>, (size_t)2 * kSmallSolveMax * kSsStride * sizeof(double)));
     small_solve_kernel<false><<<1, kSmallSolveMax, (size_t)2 * n * kSsStride * sizeof(double), stream>>>(
-        w, ldw, (int)n, perm, b, (int)k, x, status);
+        w, ldw, (int)n, perm, b, (int)k, x, status, nullptr, 0, nullptr);
   }
   RM_LAUNCHED();
   return RM_OK;
@@ -613,7 +644,8 @@ static bool cluster_lu_ok() {
 }
 
 // n <= kClusterLuMax in one launch: C CTAs (the least power of two giving at most 32 rows each).
-static int launch_cluster_lu(double* w, int64_t ldw, int n, int64_t* ipiv, int64_t* perm, cudaStream_t stream) {
+static int launch_cluster_lu(const double* a, int64_t lda, double* w, int64_t ldw, int n, int64_t* ipiv, int64_t* perm,
+                             double* amax, cudaStream_t stream) {
   const int need = (n + kClusterLuRows - 1) / kClusterLuRows;
   int C = 1;
   while (C < need) C *= 2;
@@ -631,7 +663,7 @@ static int launch_cluster_lu(double* w, int64_t ldw, int n, int64_t* ipiv, int64
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  RM_CUDA_TRY(cudaLaunchKernelEx(&cfg, cluster_lu_kernel, w, ldw, n, R, ld, ipiv, perm));
+  RM_CUDA_TRY(cudaLaunchKernelEx(&cfg, cluster_lu_kernel, a, lda, w, ldw, n, R, ld, ipiv, perm, amax));
   note_launch();
   return RM_OK;
 }
@@ -721,7 +753,7 @@ int getrf_f64(double* w, int64_t ldw, int64_t n64, int64_t* ipiv, int64_t* perm,
   if (n64 <= 0) return RM_OK;
   if (n64 > INT32_MAX / 2) return RM_BAD_ARG;
   const int n = (int)n64;
-  if (n <= kClusterLuMax && cluster_lu_ok()) return launch_cluster_lu(w, ldw, n, ipiv, perm, caller);
+  if (n <= kClusterLuMax && cluster_lu_ok()) return launch_cluster_lu(w, ldw, w, ldw, n, ipiv, perm, nullptr, caller);
   GetrfScratch* gs = reinterpret_cast<GetrfScratch*>(scratch);
   int* counters = reinterpret_cast<int*>(gs + 1);
   iota_kernel<<<std::max(1, std::min(n / 256 + 1, 1024)), 256, 0, caller>>>(perm, n);
@@ -798,6 +830,32 @@ int getrf_f64(double* w, int64_t ldw, int64_t n64, int64_t* ipiv, int64_t* perm,
     RM_CUDA_TRY(cudaStreamWaitEvent(caller, la.entry, 0));
   }
   return RM_OK;
+}
+
+// The whole plain solve of a small system in two launches: a into W factored, then the solves, the
+// regular test and the results (in page-locked host memory, complete once the stream has
+// synchronised). False when the size or the device does not take it. Copying a into W, the regular
+// test and reading two words back were three more launches and two copies, about half of the time of
+// a solve at n = 8.
+bool small_plain_solve_f64(const double* a, double* w, int64_t ldw, int64_t n, const double* b, int64_t k, double* x,
+                           int64_t* ipiv, int64_t* perm, double* amax, unsigned* status, SmallSolveResults* results,
+                           cudaStream_t stream, int* st) {
+  if (!small_solve_fits(n, k) || !cluster_lu_ok()) return false;
+  *st = launch_cluster_lu(a, n, w, ldw, (int)n, ipiv, perm, amax, stream);
+  if (*st != RM_OK) return true;
+  *st = smem_attribute(small_solve_kernel<false>, (size_t)2 * kSmallSolveMax * kSsStride * sizeof(double));
+  if (*st != RM_OK) return true;
+  int parts = 1;  // CTAs of the cluster
+  while (parts * kClusterLuRows < (int)n) parts *= 2;
+  small_solve_kernel<false><<<1, kSmallSolveMax, (size_t)2 * n * kSsStride * sizeof(double), stream>>>(
+      w, ldw, (int)n, perm, b, (int)k, x, status, amax, parts, results);
+  note_launch();
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    set_last_error(e, "small_solve_kernel", __FILE__, __LINE__);
+    *st = RM_CUDA_ERROR;
+  }
+  return true;
 }
 
 // ------------------------------------------------------------------ load / store / regular

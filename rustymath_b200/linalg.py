@@ -160,9 +160,10 @@ def _solve_one(a, b, method, report):
     torch = _torch()
     n, k = a.shape[-1], b.shape[-1]
     x = torch.empty((n, k), dtype=torch.float64, device=a.device)
-    rep = SolveReport()
+    rep = SolveReport() if report is not None else None  # asked for: the plain method forms a residual for it
     opts = _options(method)
-    st = _lib.load().rm_dsolve(n, _ptr(a), _ptr(b), k, _ptr(x), ctypes.byref(opts), ctypes.byref(rep), _stream())
+    st = _lib.load().rm_dsolve(n, _ptr(a), _ptr(b), k, _ptr(x), ctypes.byref(opts),
+                               None if rep is None else ctypes.byref(rep), _stream())
     check(st, "solve")
     if report is not None:
         report.append(rep)
