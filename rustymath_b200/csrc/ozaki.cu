@@ -27,18 +27,24 @@
 namespace rm {
 namespace oz {
 
-constexpr int BM = 128, BN = 128, BK = 128;  // BK int8 = 128 bytes: one swizzle row
-constexpr int TILE_BYTES = BM * BK;          // 16 KB per operand tile
-constexpr int STAGES = 5;
-constexpr int STAGE_BYTES = 2 * TILE_BYTES;
-constexpr int THREADS = 192;                 // TMA warp, MMA warp, 4 epilogue warps
-constexpr uint32_t TMEM_COLS = 256;          // two accumulators of BN columns
-constexpr int STG = 33;                      // epilogue staging: 32 x 33 doubles per warp
-constexpr size_t SMEM = 1024 + (size_t)STAGES * STAGE_BYTES + 4 * 32 * STG * 8 + 512;
+constexpr int BM = 128, BK = 128;            // BK int8 = 128 bytes: one swizzle row
+constexpr int A_BYTES = BM * BK;             // 16 KB
+constexpr int EPI_WARPS = 8;                 // two per TMEM lane quarter, half the columns each
+constexpr int THREADS = 64 + 32 * EPI_WARPS; // TMA warp, MMA warp, epilogue warps
+constexpr int STG = 33;                      // epilogue staging: 32 x 33 int32 per warp
+constexpr int STG_BYTES = EPI_WARPS * 32 * STG * 4;
+constexpr int kPadN = 128;                   // B's planes are padded to whole 128-row tiles
+template <int BN>
+struct Tile {
+  static constexpr int kStages = BN == 256 ? 4 : 6;
+  static constexpr int kStageBytes = A_BYTES + BN * BK;
+  static constexpr uint32_t kTmemCols = 2 * BN;  // two accumulators: orders d and d - 1
+  static constexpr size_t kSmem = 1024 + (size_t)kStages * kStageBytes + STG_BYTES + 512;
+};
 constexpr int MAX_SLICES = 8;
 
 // Instruction descriptor, kind::i8: D s32, A and B signed int8, both K-major.
-constexpr uint32_t idesc_i8(int m, int n) {
+__host__ __device__ constexpr uint32_t idesc_i8(int m, int n) {
   return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
@@ -144,45 +150,63 @@ __device__ __forceinline__ void tile_coords(int t, int ntm, int ntn, int& tm, in
   tn = in / rows;
 }
 
-// One order d of the split product over k-range [k0, k0 + kc):
-//   C (+)= 2^(ea[i] + eb[j] - 7(d+2)) sum_{p+q=d} A_p B_q^T
-// Persistent: warp 0 loads the slice tiles by TMA (rows p*mp + m0 of A's planes, q*np + n0 of
-// B's), warp 1 issues kind::i8 MMAs into one of two TMEM accumulators per tile, warps 2..5
-// drain them (int32 -> float64, scaled, added to C in coalesced rows through shared memory).
+// 2^e for -1022 <= e <= 1023
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
+// 2^e v for an integer |v| < 2^31 and any e: the first factor keeps the product exact, the
+// second rounds (or underflows, or overflows) once
+__device__ __forceinline__ double scale_any(double v, int e) {
+  const int e1 = min(max(e, -1000), 1000);
+  return v * pow2(e1) * pow2(min(max(e - e1, -1022), 1023));
+}
+
+// Orders d and (TWO) d - 1 of the split product over the k-range [k0, k0 + kc):
+//   C (+)= 2^(ea[i] + eb[j] - 7(d+2)) sum_{p+q=d} A_p B_q^T, then the same of d - 1.
+// Persistent: warp 0 loads slice tiles by TMA (rows p*mp + m0 of A's planes, q*np + n0 of
+// B's), warp 1 issues kind::i8 MMAs, warps 2..9 drain the accumulators (int32 -> float64,
+// scaled, added to C in coalesced rows through shared memory).
+//
+// An SM reads about 64 bytes a cycle from L2 and 128 from shared memory, and an int8 tile
+// product 128 x N x 128 takes 2 N cycles. One order at a time on 128 x 128 tiles loads 32 KB
+// for 256 cycles: twice what L2 delivers (the tensor pipe stood at 48%). Here a stage holds
+// A_p and B_{d-p}, and B_{d-p} also meets the A_{p-1} of the stage before it for the order
+// d - 1, so a loaded tile is used twice; with N = 256 that is 48 KB for 1024 cycles. Both
+// accumulators take all 512 TMEM columns, so the epilogue is not overlapped with the tile's
+// successor; it is under 3% of the 2d + 1 products, and C is read and written half as often.
+// 8192^3, 8 slices, the whole call: 22.7 ms before, 15.2 after.
+template <int BN, bool TWO>
 __global__ void __launch_bounds__(THREADS, 1)
     ozaki_order_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                        double* __restrict__ c, int64_t ldc, int m, int n, int mp, int np, int k0, int kc, int d,
                        const int* __restrict__ ea, const int* __restrict__ eb, int first, unsigned* status) {
+  using T = Tile<BN>;
+  constexpr int STAGES = T::kStages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  double* stg_all = reinterpret_cast<double*>(smem + STAGES * STAGE_BYTES);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES + 4 * 32 * STG * 8);
+  int* stg_all = reinterpret_cast<int*>(smem + STAGES * T::kStageBytes);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * T::kStageBytes + STG_BYTES);
   uint64_t* empty = full + STAGES;
   uint64_t* tfull = empty + STAGES;
-  uint64_t* tempty = tfull + 2;
-  uint64_t* mma_done = tempty + 2;
+  uint64_t* tempty = tfull + 1;
+  uint64_t* mma_done = tempty + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_done + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ntn = (n + BN - 1) / BN, ntm = (m + BM - 1) / BM;
   const int tiles = ntm * ntn;
   const int ktiles = (kc + BK - 1) / BK;
-  const int pairs = d + 1;  // (p, d - p) for p = 0..d
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&tfull[b], 1);
-      mbar_init(&tempty[b], 4);
-    }
+    mbar_init(tfull, 1);
+    mbar_init(tempty, EPI_WARPS);
     mbar_init(mma_done, 1);
     fence_barrier_init();
   }
   if (warp == 1) {
-    tc::tmem_alloc(tmem_slot, TMEM_COLS);
+    tc::tmem_alloc(tmem_slot, T::kTmemCols);
     tc::fence_before();
   }
   __syncthreads();
@@ -199,17 +223,17 @@ __global__ void __launch_bounds__(THREADS, 1)
         int tmi, tni;
         tile_coords(tile, ntm, ntn, tmi, tni);
         const int m0 = tmi * BM, n0 = tni * BN;
-        for (int pq = 0; pq < pairs && ok; ++pq)
-          for (int kt = 0; kt < ktiles; ++kt, ++it) {
+        for (int kt = 0; kt < ktiles && ok; ++kt)
+          for (int p = 0; p <= d; ++p, ++it) {
             const int s = it % STAGES;
             if (!mbar_wait(&empty[s], ((it / STAGES) & 1u) ^ 1u, status)) {
               ok = false;
               break;
             }
-            uint8_t* st = smem + s * STAGE_BYTES;
-            mbar_arrive_expect_tx(&full[s], STAGE_BYTES);
-            tma_load_2d(st, &tm_a, &full[s], k0 + kt * BK, pq * mp + m0);
-            tma_load_2d(st + TILE_BYTES, &tm_b, &full[s], k0 + kt * BK, (d - pq) * np + n0);
+            uint8_t* st = smem + s * T::kStageBytes;
+            mbar_arrive_expect_tx(&full[s], T::kStageBytes);
+            tma_load_2d(st, &tm_a, &full[s], k0 + kt * BK, p * mp + m0);
+            tma_load_2d(st + A_BYTES, &tm_b, &full[s], k0 + kt * BK, (d - p) * np + n0);
           }
       }
       for (int j = (it > STAGES ? it - STAGES : 0); j < it; ++j) mbar_wait(&full[j % STAGES], (j / STAGES) & 1u, status);
@@ -217,93 +241,138 @@ __global__ void __launch_bounds__(THREADS, 1)
   } else if (warp == 1) {
     if (lane == 0) {
       constexpr uint32_t idesc = idesc_i8(BM, BN);
-      int it = 0, lt = 0;
+      const uint32_t base = smem_u32(smem);
+      int it = 0, lt = 0, prev = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++lt) {
-        const int buf = lt & 1;
-        if (!mbar_wait(&tempty[buf], ((lt >> 1) & 1u) ^ 1u, status)) break;
+        if (!mbar_wait(tempty, (lt & 1u) ^ 1u, status)) break;
         tc::fence_after();
-        const uint32_t dt = tmem + buf * BN;
-        for (int pq = 0; pq < pairs && ok; ++pq)
-          for (int kt = 0; kt < ktiles; ++kt, ++it) {
+        for (int kt = 0; kt < ktiles && ok; ++kt)
+          for (int p = 0; p <= d; ++p, ++it) {
             const int s = it % STAGES;
             if (!mbar_wait(&full[s], (it / STAGES) & 1u, status)) {
               ok = false;
               break;
             }
             tc::fence_after();
-            const uint32_t sa = smem_u32(smem + s * STAGE_BYTES), sb = sa + TILE_BYTES;
+            const uint32_t sa = base + s * T::kStageBytes, sb = sa + A_BYTES;
 #pragma unroll
-            for (int kk = 0; kk < BK / 32; ++kk) {  // K = 32 int8 = 32 bytes per MMA
-              const uint32_t acc = (pq == 0 && kt == 0 && kk == 0) ? 0u : 1u;
-              mma_i8(dt, tc::smem_desc(sa + kk * 32), tc::smem_desc(sb + kk * 32), idesc, acc);
+            for (int kk = 0; kk < BK / 32; ++kk)  // K = 32 int8 = 32 bytes per MMA
+              mma_i8(tmem, tc::smem_desc(sa + kk * 32), tc::smem_desc(sb + kk * 32), idesc,
+                     (kt == 0 && p == 0 && kk == 0) ? 0u : 1u);
+            if (TWO && p > 0) {
+              const uint32_t sp = base + prev * T::kStageBytes;
+#pragma unroll
+              for (int kk = 0; kk < BK / 32; ++kk)
+                mma_i8(tmem + BN, tc::smem_desc(sp + kk * 32), tc::smem_desc(sb + kk * 32), idesc,
+                       (kt == 0 && p == 1 && kk == 0) ? 0u : 1u);
+              tc::mma_commit(&empty[prev]);
             }
-            tc::mma_commit(&empty[s]);
+            if (!TWO || p == d) tc::mma_commit(&empty[s]);
+            prev = s;
           }
-        if (ok) tc::mma_commit(&tfull[buf]);
+        if (ok) tc::mma_commit(tfull);
       }
       tc::mma_commit(mma_done);
       mbar_wait(mma_done, 0u, status);
     }
   } else {
-    // epilogue: warps 2..5, TMEM lane quarter warp % 4
-    const int q = warp & 3;
-    double* stg = stg_all + (warp - 2) * 32 * STG;
+    // epilogue: warps 2..9, TMEM lane quarter warp % 4, half of the columns
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    int* stg = stg_all + (warp - 2) * 32 * STG;
     int lt = 0;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++lt) {
-      const int buf = lt & 1;
-      if (!mbar_wait(&tfull[buf], (lt >> 1) & 1u, status)) break;
-      tc::fence_after();
       int tmi, tni;
       tile_coords(tile, ntm, ntn, tmi, tni);
-      const int m0 = tmi * BM, n0 = tni * BN;
-      const int row0 = m0 + q * 32;
+      const int row0 = tmi * BM + q * 32;
+      const int er = row0 + lane < m ? ea[row0 + lane] : 0;
+      const int ermin = __reduce_min_sync(0xffffffffu, er), ermax = __reduce_max_sync(0xffffffffu, er);
+      const uint32_t tq = tmem + ((uint32_t)(q * 32) << 16);
+      bool waited = false;
 #pragma unroll 1
-      for (int cb = 0; cb < BN; cb += 32) {
-        uint32_t v[32];
-        tc::tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + buf * BN + cb, v);
-        if (cb == BN - 32) {
-          tc::fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&tempty[buf]);
-        }
-        __syncwarp();
-#pragma unroll
-        for (int j = 0; j < 32; ++j) stg[lane * STG + j] = (double)(int)v[j];
-        __syncwarp();
-        const int col = n0 + cb + lane;
-        const int ecol = col < n ? eb[col] : 0;
+      for (int cb = half * (BN / 2); cb < (half + 1) * (BN / 2); cb += 32) {
+        const int col = tni * BN + cb + lane;
         double cv[32];
-        if (!first) {
 #pragma unroll
-          for (int rr = 0; rr < 32; ++rr) {
-            const int row = row0 + rr;
-            cv[rr] = (row < m && col < n) ? c[(int64_t)row * ldc + col] : 0.0;
+        for (int rr = 0; rr < 32; ++rr)
+          cv[rr] = (!first && row0 + rr < m && col < n) ? c[(int64_t)(row0 + rr) * ldc + col] : 0.0;
+        const int ecol = (col < n ? eb[col] : 0) - 7 * (d + 2);
+        const bool plain = __all_sync(0xffffffffu, ermin + ecol >= -1022 && ermax + ecol + 7 <= 1023);
+        if (!waited) {  // after the first chunk of C has been asked for
+          if (!__all_sync(0xffffffffu, mbar_wait(tfull, lt & 1u, status))) goto out;
+          tc::fence_after();
+          waited = true;
+        }
+#pragma unroll
+        for (int o = 0; o < (TWO ? 2 : 1); ++o) {
+          uint32_t v[32];
+          tc::tmem_ld32(tq + o * BN + cb, v);
+          if (o == (TWO ? 1 : 0) && cb == (half + 1) * (BN / 2) - 32) {
+            tc::fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(tempty);
+          }
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) stg[lane * STG + j] = (int)v[j];
+          __syncwarp();
+          if (plain) {
+#pragma unroll
+            for (int rr = 0; rr < 32; ++rr)
+              cv[rr] += (double)stg[rr * STG + lane] * pow2(__shfl_sync(0xffffffffu, er, rr) + ecol + 7 * o);
+          } else {
+#pragma unroll
+            for (int rr = 0; rr < 32; ++rr)
+              cv[rr] += scale_any((double)stg[rr * STG + lane], __shfl_sync(0xffffffffu, er, rr) + ecol + 7 * o);
           }
         }
 #pragma unroll
-        for (int rr = 0; rr < 32; ++rr) {
-          const int row = row0 + rr;
-          if (row < m && col < n) {
-            const double val = ldexp(stg[rr * STG + lane], ea[row] + ecol - 7 * (d + 2));
-            c[(int64_t)row * ldc + col] = first ? val : cv[rr] + val;
-          }
-        }
+        for (int rr = 0; rr < 32; ++rr)
+          if (row0 + rr < m && col < n) c[(int64_t)(row0 + rr) * ldc + col] = cv[rr];
       }
     }
+  out:;
   }
   tc::fence_before();
   __syncthreads();
   if (warp == 1) {
     tc::fence_after();
-    tc::tmem_free(tmem, TMEM_COLS);
+    tc::tmem_free(tmem, T::kTmemCols);
   }
+}
+
+// Every order of every k chunk, the smallest terms first, two orders to a launch
+template <int BN>
+int orders(int64_t m, int64_t n, int64_t k, double* c, int64_t ldc, int s, const int8_t* asl, const int8_t* bsl,
+           int64_t mp, int64_t np, int64_t kp, int64_t kmax, const int* ea, const int* eb, unsigned* status,
+           cudaStream_t stream) {
+  constexpr size_t smem = Tile<BN>::kSmem;
+  RM_TRY(smem_attribute(ozaki_order_kernel<BN, true>, smem));
+  RM_TRY(smem_attribute(ozaki_order_kernel<BN, false>, smem));
+  CUtensorMap ta, tb;
+  RM_TRY(make_tensor_map_2d(&ta, asl, 1, kp, s * mp, kp, BK, BM, true));
+  // a 256-row box may reach into the next plane or past the last one: columns beyond n, not stored
+  RM_TRY(make_tensor_map_2d(&tb, bsl, 1, kp, s * np, kp, BK, BN, true));
+  const int64_t tiles = (mp / BM) * ((n + BN - 1) / BN);
+  const unsigned grid = (unsigned)std::min<int64_t>(tiles, device_sm_count());
+  int first = 1;
+  for (int64_t k0 = 0; k0 < k; k0 += kmax) {
+    const int kc = (int)std::min<int64_t>(kmax, k - k0);
+    for (int d = s - 1; d >= 0; d -= 2) {
+      auto kernel = d > 0 ? ozaki_order_kernel<BN, true> : ozaki_order_kernel<BN, false>;
+      kernel<<<grid, THREADS, smem, stream>>>(ta, tb, c, ldc, (int)m, (int)n, (int)mp, (int)np, (int)k0, kc, d, ea, eb,
+                                              first, status);
+      RM_LAUNCHED();
+      first = 0;
+    }
+  }
+  return RM_OK;
 }
 
 }  // namespace oz
 
 size_t ozaki_scratch_bytes(int64_t m, int64_t n, int64_t k, int s) {
-  const int64_t mp = (m + oz::BM - 1) / oz::BM * oz::BM, np = (n + oz::BN - 1) / oz::BN * oz::BN;
+  const int64_t mp = (m + oz::BM - 1) / oz::BM * oz::BM, np = (n + oz::kPadN - 1) / oz::kPadN * oz::kPadN;
   const int64_t kp = (k + oz::BK - 1) / oz::BK * oz::BK;
   return (size_t)s * (mp + np) * kp + (size_t)(m + n) * sizeof(int) + 1024;
 }
@@ -321,13 +390,12 @@ int dgemm_ozaki(int64_t m, int64_t n, int64_t k, const double* a, int64_t lda, c
     RM_CUDA_TRY(cudaMemset2DAsync(c, ldc * sizeof(double), 0, n * sizeof(double), m, stream));
     return RM_OK;
   }
-  const int64_t mp = (m + oz::BM - 1) / oz::BM * oz::BM, np = (n + oz::BN - 1) / oz::BN * oz::BN;
+  const int64_t mp = (m + oz::BM - 1) / oz::BM * oz::BM, np = (n + oz::kPadN - 1) / oz::kPadN * oz::kPadN;
   const int64_t kp = (k + oz::BK - 1) / oz::BK * oz::BK;
   int8_t* asl = reinterpret_cast<int8_t*>(scratch);
   int8_t* bsl = asl + (size_t)s * mp * kp;
   int* ea = reinterpret_cast<int*>(bsl + (size_t)s * np * kp);
   int* eb = ea + m;
-  RM_TRY(smem_attribute(oz::ozaki_order_kernel, oz::SMEM));
   const int mi = (int)m, ni = (int)n, ki = (int)k;
   // exponents and slices (the padding of the planes stays zero)
   RM_CUDA_TRY(cudaMemsetAsync(asl, 0, (size_t)s * (mp + np) * kp, stream));
@@ -346,24 +414,18 @@ int dgemm_ozaki(int64_t m, int64_t n, int64_t k, const double* a, int64_t lda, c
   oz::split_cols_kernel<<<dim3((unsigned)((n + 31) / 32), (unsigned)((k + 31) / 32)), dim3(32, 8), 0, stream>>>(
       b, ldb, ki, ni, eb, s, bsl, kp, np * kp);
   RM_LAUNCHED();
-  CUtensorMap ta, tb;
-  RM_TRY(make_tensor_map_2d(&ta, asl, 1, kp, s * mp, kp, oz::BK, oz::BM, true));
-  RM_TRY(make_tensor_map_2d(&tb, bsl, 1, kp, s * np, kp, oz::BK, oz::BN, true));
   // k chunks short enough that an order's int32 sums cannot overflow: s k 127^2 < 2^31
   const int64_t kmax = std::max<int64_t>(oz::BK, ((int64_t)INT_MAX / ((int64_t)s * 127 * 127)) / oz::BK * oz::BK);
-  const int64_t tiles = (mp / oz::BM) * (np / oz::BN);
-  const unsigned grid = (unsigned)std::min<int64_t>(tiles, device_sm_count());
-  bool first = true;
-  for (int64_t k0 = 0; k0 < k; k0 += kmax) {
-    const int kc = (int)std::min<int64_t>(kmax, k - k0);
-    for (int d = s - 1; d >= 0; --d) {  // the smallest terms first
-      oz::ozaki_order_kernel<<<grid, oz::THREADS, oz::SMEM, stream>>>(ta, tb, c, ldc, mi, ni, (int)mp, (int)np,
-                                                                     (int)k0, kc, d, ea, eb, first ? 1 : 0, status);
-      RM_LAUNCHED();
-      first = false;
-    }
-  }
-  return RM_OK;
+  // 128 x 256 tiles need less traffic per product, 128 x 128 tiles spread a small product over
+  // more SMs: by the waves that each takes, a wide tile costing two narrow ones over 1.3 (wide
+  // against narrow, us: 1300 x 1300, k = 1024, one wave of either, 221 : 172; 1700 x 1400,
+  // k = 1700, one : two, 319 : 402; 2200 x 2200, k = 1000, two : three, 418 : 399; 2500 x 2500,
+  // k = 3000, 896 : 926; 3500^3, three : six, 1477 : 2007; 8192^3 14.2 : 19.3 ms)
+  const int64_t sms = device_sm_count();
+  const int64_t narrow = (mp / oz::BM) * ((n + 127) / 128), wide = (mp / oz::BM) * ((n + 255) / 256);
+  const bool use_wide = 20 * ((wide + sms - 1) / sms) <= 13 * ((narrow + sms - 1) / sms);
+  return use_wide ? oz::orders<256>(m, n, k, c, ldc, s, asl, bsl, mp, np, kp, kmax, ea, eb, status, stream)
+                  : oz::orders<128>(m, n, k, c, ldc, s, asl, bsl, mp, np, kp, kmax, ea, eb, status, stream);
 }
 
 }  // namespace rm
