@@ -63,17 +63,6 @@ __device__ __forceinline__ int exponent_of(double v) {
   return e;
 }
 
-// ea[i] for each row of the m x k row-major a: a warp per row
-__global__ void row_exponent_kernel(const double* __restrict__ a, int64_t lda, int m, int k, int* __restrict__ ea) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= m) return;
-  int e = INT_MIN;
-  for (int j = lane; j < k; j += 32) e = max(e, exponent_of(fabs(a[(int64_t)warp * lda + j])));
-#pragma unroll
-  for (int off = 16; off; off >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, off));
-  if (lane == 0) ea[warp] = e == INT_MIN ? 0 : e;
-}
-
 // eb[j] (pre-set to INT_MIN) for each column of the k x n row-major b: 32 x 32 tiles, atomics
 __global__ void col_exponent_kernel(const double* __restrict__ b, int64_t ldb, int k, int n, int* __restrict__ eb) {
   __shared__ int cm[32];
@@ -94,46 +83,101 @@ __global__ void fix_exponent_kernel(int* e, int n) {
   if (i < n && e[i] == INT_MIN) e[i] = 0;
 }
 
-// The s slices of row i of a (scaled by 2^-ea[i]) into planes [p][i][kk] (row stride kp,
-// plane stride mp * kp): a warp per row, lanes along it.
-__global__ void split_rows_kernel(const double* __restrict__ a, int64_t lda, int m, int k, const int* __restrict__ ea,
-                                  int s, int8_t* __restrict__ out, int64_t kp, int64_t plane) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= m) return;
-  const int e = ea[warp];
-  for (int j = lane; j < k; j += 32) {
-    double r = ldexp(a[(int64_t)warp * lda + j], -e);
+// 2^e for -1022 <= e <= 1023
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
+
+// The s signed base-128 digits of 2^-e x, truncated toward zero, the first in the low byte. For
+// a finite |2^-e x| < 1 they are those of one fixed-point number of 7 s bits, which costs one
+// conversion where a digit at a time costs two roundings each; the rest (a row or column with
+// an infinity) goes digit by digit.
+__device__ __forceinline__ uint64_t digits(double x, int e, int s) {
+  const double r = (unsigned)(e + 1022) <= 2044u ? x * pow2(-e) : ldexp(x, -e);
+  uint64_t out = 0;
+  if (fabs(r) < 1.0) {
+    uint64_t v = (uint64_t)__double2ll_rz(fabs(r) * pow2(7 * s));
+    const uint64_t neg = r < 0.0 ? 0xff : 0;
+    for (int p = s - 1; p >= 0; --p, v >>= 7) out |= ((((v & 127) ^ neg) - neg) & 0xff) << (8 * p);
+  } else {
+    double t = r;
     for (int p = 0; p < s; ++p) {
-      r *= 128.0;
-      const double t = trunc(r);
-      r -= t;
-      out[p * plane + (int64_t)warp * kp + j] = (int8_t)t;
+      t *= 128.0;
+      const double d = trunc(t);
+      t -= d;
+      out |= (uint64_t)(uint8_t)(int8_t)d << (8 * p);
     }
+  }
+  return out;
+}
+
+// Byte p of four words of digits, the first word's lowest
+__device__ __forceinline__ uint32_t plane_word(const uint64_t (&w)[4], int p) {
+  const int sh = 8 * p;
+  return (uint32_t)((w[0] >> sh) & 0xff) | (uint32_t)((w[1] >> sh) & 0xff) << 8 |
+         (uint32_t)((w[2] >> sh) & 0xff) << 16 | (uint32_t)((w[3] >> sh) & 0xff) << 24;
+}
+
+// ea[i] and the s slices of row i of a into planes [p][i][kk] (row stride kp, plane stride
+// mp * kp), zero from k to kp: a block per row, so that the second pass over the row finds it
+// in L2, and four columns a lane, so that a warp's stores are 128 bytes in each plane. Rows
+// from m to mp stay unwritten: they only meet rows of C that are not stored.
+__global__ void __launch_bounds__(256)
+    split_rows_kernel(const double* __restrict__ a, int64_t lda, int k, int* __restrict__ ea, int s,
+                      int8_t* __restrict__ out, int64_t kp, int64_t plane) {
+  __shared__ int part[8];
+  const int64_t row = blockIdx.x;
+  const double* ar = a + row * lda;
+  int e = INT_MIN;
+#pragma unroll 4
+  for (int j = threadIdx.x; j < k; j += 256) e = max(e, exponent_of(fabs(ar[j])));
+  e = __reduce_max_sync(0xffffffffu, e);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = e;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < 8; ++w) e = max(e, part[w]);
+  if (e == INT_MIN) e = 0;
+  if (threadIdx.x == 0) ea[row] = e;
+  for (int64_t j = 4 * threadIdx.x; j < kp; j += 1024) {
+    double x[4];
+    uint64_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = j + i < k ? ar[j + i] : 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = digits(x[i], e, s);
+    for (int p = 0; p < s; ++p)
+      *reinterpret_cast<uint32_t*>(out + p * plane + row * kp + j) = plane_word(w, p);
   }
 }
 
 // The s slices of column j of b (scaled by 2^-eb[j]), transposed: planes [q][j][kk] (row
-// stride kp). 32 x 32 tiles through shared memory: reads along b's rows, writes along k.
-__global__ void split_cols_kernel(const double* __restrict__ b, int64_t ldb, int k, int n, const int* __restrict__ eb,
-                                  int s, int8_t* __restrict__ out, int64_t kp, int64_t plane) {
-  __shared__ int8_t t8[MAX_SLICES][32][33];
-  const int r0 = blockIdx.y * 32, j0 = blockIdx.x * 32;
-  const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
-  for (int rr = ty; rr < 32; rr += 8) {
-    const int r = r0 + rr, j = j0 + tx;
-    double v = (r < k && j < n) ? ldexp(b[(int64_t)r * ldb + j], -eb[j]) : 0.0;
-    for (int q = 0; q < s; ++q) {
-      v *= 128.0;
-      const double t = trunc(v);
-      v -= t;
-      t8[q][tx][rr] = (int8_t)t;
+// stride kp). A block takes 128 rows and 32 columns through shared memory: reads along b's
+// rows, four of them a thread, and 128-byte stores along k. What lies past k meets A's zeros,
+// so nothing else of the planes is written.
+__global__ void __launch_bounds__(256)
+    split_cols_kernel(const double* __restrict__ b, int64_t ldb, int k, int n, const int* __restrict__ eb, int s,
+                      int8_t* __restrict__ out, int64_t kp, int64_t plane) {
+  __shared__ uint32_t t8[MAX_SLICES][32][33];
+  const int r0 = blockIdx.y * 128, j0 = blockIdx.x * 32;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int j = j0 + tx;
+  const int e = j < n ? eb[j] : 0;
+#pragma unroll
+  for (int g = ty; g < 32; g += 8) {
+    double x[4];
+    uint64_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = r0 + 4 * g + i;
+      x[i] = (r < k && j < n) ? b[(int64_t)r * ldb + j] : 0.0;
     }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = digits(x[i], e, s);
+    for (int q = 0; q < s; ++q) t8[q][tx][g] = plane_word(w, q);
   }
   __syncthreads();
-  for (int jj = ty; jj < 32; jj += 8) {
-    const int j = j0 + jj, r = r0 + tx;
-    if (j < n && r < k)
-      for (int q = 0; q < s; ++q) out[q * plane + (int64_t)j * kp + r] = t8[q][jj][tx];
+  for (int i = ty; i < 32 * s; i += 8) {
+    const int q = i >> 5, jj = i & 31;
+    if (j0 + jj < n)
+      *reinterpret_cast<uint32_t*>(out + q * plane + (int64_t)(j0 + jj) * kp + r0 + 4 * tx) = t8[q][jj][tx];
   }
 }
 
@@ -150,8 +194,6 @@ __device__ __forceinline__ void tile_coords(int t, int ntm, int ntn, int& tm, in
   tn = in / rows;
 }
 
-// 2^e for -1022 <= e <= 1023
-__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
 // 2^e v for an integer |v| < 2^31 and any e: the first factor keeps the product exact, the
 // second rounds (or underflows, or overflows) once
 __device__ __forceinline__ double scale_any(double v, int e) {
@@ -396,10 +438,10 @@ int dgemm_ozaki(int64_t m, int64_t n, int64_t k, const double* a, int64_t lda, c
   int8_t* bsl = asl + (size_t)s * mp * kp;
   int* ea = reinterpret_cast<int*>(bsl + (size_t)s * np * kp);
   int* eb = ea + m;
-  const int mi = (int)m, ni = (int)n, ki = (int)k;
-  // exponents and slices (the padding of the planes stays zero)
-  RM_CUDA_TRY(cudaMemsetAsync(asl, 0, (size_t)s * (mp + np) * kp, stream));
-  oz::row_exponent_kernel<<<(unsigned)((m * 32 + 255) / 256), 256, 0, stream>>>(a, lda, mi, ki, ea);
+  const int ni = (int)n, ki = (int)k;
+  // exponents and slices; int8 planes hold no value that could spread, so only A's columns from
+  // k to kp are cleared
+  oz::split_rows_kernel<<<(unsigned)m, 256, 0, stream>>>(a, lda, ki, ea, s, asl, kp, mp * kp);
   RM_LAUNCHED();
   fill_int_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(eb, ni, INT_MIN);
   RM_LAUNCHED();
@@ -408,10 +450,7 @@ int dgemm_ozaki(int64_t m, int64_t n, int64_t k, const double* a, int64_t lda, c
   RM_LAUNCHED();
   oz::fix_exponent_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(eb, ni);
   RM_LAUNCHED();
-  oz::split_rows_kernel<<<(unsigned)((m * 32 + 255) / 256), 256, 0, stream>>>(a, lda, mi, ki, ea, s, asl, kp,
-                                                                               mp * kp);
-  RM_LAUNCHED();
-  oz::split_cols_kernel<<<dim3((unsigned)((n + 31) / 32), (unsigned)((k + 31) / 32)), dim3(32, 8), 0, stream>>>(
+  oz::split_cols_kernel<<<dim3((unsigned)((n + 31) / 32), (unsigned)(kp / 128)), 256, 0, stream>>>(
       b, ldb, ki, ni, eb, s, bsl, kp, np * kp);
   RM_LAUNCHED();
   // k chunks short enough that an order's int32 sums cannot overflow: s k 127^2 < 2^31
