@@ -22,7 +22,11 @@ static_assert(NMAX == MAX_N, "the build's size class");
 constexpr int THREADS = NMAX;
 constexpr int WARPS = THREADS / 32;
 constexpr int KMAX = kBatchMaxK;
-constexpr int SLOT_BYTES = 144;
+// The 64-thread build takes its pivots by integer keys with the reciprocals posted, and float
+// reciprocals by approximation: those systems are bound by the latency of a column. In the 256-thread
+// build the same changes made the kernel's code longer and every phase ~8% slower, so it keeps its own.
+constexpr bool SHORT = NMAX <= 64;
+constexpr int SLOT_BYTES = SHORT ? 160 : 144;
 constexpr int UBT_BYTES = NMAX * 144;  // U12 transposed (NMAX rows of 144 bytes), or row segments
 
 struct Smem {
@@ -106,12 +110,48 @@ __device__ __forceinline__ T tabs(T v) {
   return v < T(0) ? -v : v;
 }
 
+// The reciprocal that rustymath's divide multiplies by; 0 where a pivot is divided by instead (a
+// subnormal one) or has a reciprocal that rounds to 0. float: the hardware's approximation and two
+// Newton steps x += x (1 - a x), the second of which rounds correctly but for a mantissa of all
+// ones (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor",
+// 1990): no branch, where the intrinsic's ~130 cycles were on the path of every column.
+__device__ __forceinline__ double brecip(double piv) { return fabs(piv) < DBL_MIN ? 0.0 : 1.0 / piv; }
+__device__ __forceinline__ float brecip(float piv) {
+  float x;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(x) : "f"(piv));
+  const float y = fmaf(x, fmaf(-piv, x, 1.0f), x);
+  const float z = fmaf(y, fmaf(-piv, y, 1.0f), y);
+  return fabsf(piv) < FLT_MIN || x == 0.0f ? 0.0f : z;
+}
+// y / d from d's reciprocal rd: the product and one correction by its remainder (the same paper); the
+// product itself where that is no number (an infinite y)
+__device__ __forceinline__ float bquotient(float y, float d, float rd) {
+  const float q = y * rd, t = fmaf(fmaf(-q, d, y), rd, q);
+  return t != t ? q : t;
+}
 // rustymath's divide: multiply by the reciprocal unless the pivot is subnormal
 __device__ __forceinline__ double bdivide(double x, double piv) {
   return fabs(piv) < DBL_MIN ? x / piv : x * (1.0 / piv);
 }
+__device__ __noinline__ float bdivide_rare(float x, float piv) { return x / piv; }
 __device__ __forceinline__ float bdivide(float x, float piv) {
+  if constexpr (SHORT) {
+    const float r = brecip(piv);
+    return r != 0.0f ? x * r : bdivide_rare(x, piv);
+  }
   return fabsf(piv) < FLT_MIN ? x / piv : x * __frcp_rn(piv);
+}
+
+// The lowest lane of the warp's largest key (hi, lo); lo counts for T = double only.
+template <typename T>
+__device__ __forceinline__ int best_lane(unsigned hi, unsigned lo) {
+  const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
+  unsigned top = __ballot_sync(0xffffffffu, hi == mhi);
+  if (sizeof(T) == 8 && (top & (top - 1u))) {
+    const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
+    top = __ballot_sync(0xffffffffu, hi == mhi && lo == mlo);
+  }
+  return __ffs(top) - 1;
 }
 
 template <typename T>
@@ -327,51 +367,79 @@ __device__ void bfactor_pivoted(T* W, int ld, int n, Smem& sm, int& my_pos) {
     for (int c = 0; c < NB; ++c) {
       if (c < nbj) {
         unsigned char(*sl)[SLOT_BYTES] = sm.slot[c & 1];
-        T key = T(-1);
-        int idx = r, bi, bw;
-        if (sizeof(T) == 4) {
-          // float: |pivot| as an ordered 32-bit key (0 none, 1 NaN, bits + 2), redux max + ballot
-          const float v = fabsf((float)p[c]);
-          const unsigned uk = active ? (v != v ? 1u : __float_as_uint(v) + 2u) : 0u;
-          const unsigned wmax = __reduce_max_sync(0xffffffffu, uk);
-          const int wl = __ffs(__ballot_sync(0xffffffffu, uk == wmax)) - 1;
-          if (lane == wl) {
+        int bi, bw;
+        if constexpr (SHORT) {
+          // the largest magnitude, the lowest row among equals; a NaN only when nothing else is left.
+          // Keys: 0 no candidate, 1 NaN, else the magnitude's (high) bits + 2 and low bits. The
+          // reciprocal a winner would give is formed beside the reduction and posted.
+          unsigned hi = 0u, lo = 0u;
+          if constexpr (sizeof(T) == 4) {
+            const float v = fabsf(p[c]);
+            if (active) hi = v != v ? 1u : __float_as_uint(v) + 2u;
+          } else {
+            const unsigned long long m = (unsigned long long)__double_as_longlong(p[c]) & 0x7fffffffffffffffull;
+            if (active) hi = m > 0x7ff0000000000000ull ? 1u : (unsigned)(m >> 32) + 2u;
+            lo = hi > 1u ? (unsigned)m : 0u;
+          }
+          const T rcp = brecip(p[c]);
+          if (lane == best_lane<T>(hi, lo)) {
             T* post = reinterpret_cast<T*>(sl[warp]);
 #pragma unroll
             for (int i = 0; i < NB; ++i) post[i] = p[i];
-            *reinterpret_cast<unsigned*>(sl[warp] + 128) = wmax;
-            *reinterpret_cast<int*>(sl[warp] + 136) = r;
+            *reinterpret_cast<uint4*>(sl[warp] + 128) = make_uint4(hi, lo, (unsigned)r, 0u);
+            *reinterpret_cast<T*>(sl[warp] + 144) = rcp;
           }
           __syncthreads();
-          const unsigned kq = lane < WARPS ? *reinterpret_cast<const unsigned*>(sl[lane] + 128) : 0u;
-          const unsigned gmax = __reduce_max_sync(0xffffffffu, kq);
-          const unsigned gball = __ballot_sync(0xffffffffu, lane < WARPS && kq == gmax);
-          bw = gball ? __ffs(gball) - 1 : 0;
+          const uint2 post_key = lane < WARPS ? *reinterpret_cast<const uint2*>(sl[lane] + 128) : make_uint2(0u, 0u);
+          bw = best_lane<T>(post_key.x, post_key.y);  // lanes are warps, in row order
           bi = *reinterpret_cast<const int*>(sl[bw] + 136);
         } else {
-          if (active) {
-            const T v = tabs(p[c]);
-            key = v != v ? T(-0.5) : v;
-          }
-          warp_argmax(key, idx);
-          if (lane == (idx & 31)) {
-            T* post = reinterpret_cast<T*>(sl[warp]);
+          T key = T(-1);
+          int idx = r;
+          if (sizeof(T) == 4) {
+            // float: |pivot| as an ordered 32-bit key (0 none, 1 NaN, bits + 2), redux max + ballot
+            const float v = fabsf((float)p[c]);
+            const unsigned uk = active ? (v != v ? 1u : __float_as_uint(v) + 2u) : 0u;
+            const unsigned wmax = __reduce_max_sync(0xffffffffu, uk);
+            const int wl = __ffs(__ballot_sync(0xffffffffu, uk == wmax)) - 1;
+            if (lane == wl) {
+              T* post = reinterpret_cast<T*>(sl[warp]);
 #pragma unroll
-            for (int i = 0; i < NB; ++i) post[i] = p[i];
-            *reinterpret_cast<T*>(sl[warp] + 128) = key;
-            *reinterpret_cast<int*>(sl[warp] + 136) = idx;
-          }
-          __syncthreads();
-          T bk = *reinterpret_cast<const T*>(sl[0] + 128);
-          bi = *reinterpret_cast<const int*>(sl[0] + 136), bw = 0;
+              for (int i = 0; i < NB; ++i) post[i] = p[i];
+              *reinterpret_cast<unsigned*>(sl[warp] + 128) = wmax;
+              *reinterpret_cast<int*>(sl[warp] + 136) = r;
+            }
+            __syncthreads();
+            const unsigned kq = lane < WARPS ? *reinterpret_cast<const unsigned*>(sl[lane] + 128) : 0u;
+            const unsigned gmax = __reduce_max_sync(0xffffffffu, kq);
+            const unsigned gball = __ballot_sync(0xffffffffu, lane < WARPS && kq == gmax);
+            bw = gball ? __ffs(gball) - 1 : 0;
+            bi = *reinterpret_cast<const int*>(sl[bw] + 136);
+          } else {
+            if (active) {
+              const T v = tabs(p[c]);
+              key = v != v ? T(-0.5) : v;
+            }
+            warp_argmax(key, idx);
+            if (lane == (idx & 31)) {
+              T* post = reinterpret_cast<T*>(sl[warp]);
 #pragma unroll
-          for (int w = 1; w < WARPS; ++w) {
-            const T k2 = *reinterpret_cast<const T*>(sl[w] + 128);
-            const int i2 = *reinterpret_cast<const int*>(sl[w] + 136);
-            if (k2 > bk || (k2 == bk && i2 < bi)) {
-              bk = k2;
-              bi = i2;
-              bw = w;
+              for (int i = 0; i < NB; ++i) post[i] = p[i];
+              *reinterpret_cast<T*>(sl[warp] + 128) = key;
+              *reinterpret_cast<int*>(sl[warp] + 136) = idx;
+            }
+            __syncthreads();
+            T bk = *reinterpret_cast<const T*>(sl[0] + 128);
+            bi = *reinterpret_cast<const int*>(sl[0] + 136), bw = 0;
+#pragma unroll
+            for (int w = 1; w < WARPS; ++w) {
+              const T k2 = *reinterpret_cast<const T*>(sl[w] + 128);
+              const int i2 = *reinterpret_cast<const int*>(sl[w] + 136);
+              if (k2 > bk || (k2 == bk && i2 < bi)) {
+                bk = k2;
+                bi = i2;
+                bw = w;
+              }
             }
           }
         }
@@ -388,7 +456,13 @@ __device__ void bfactor_pivoted(T* W, int ld, int n, Smem& sm, int& my_pos) {
         }
         if (active) {
           if (piv != T(0)) {
-            const T l = bdivide(p[c], piv);
+            T l;
+            if constexpr (SHORT) {
+              const T r1 = *reinterpret_cast<const T*>(sl[bw] + 144);
+              l = r1 != T(0) ? p[c] * r1 : bdivide(p[c], piv);
+            } else {
+              l = bdivide(p[c], piv);
+            }
             p[c] = l;
 #pragma unroll
             for (int i = c + 1; i < NB; ++i) p[i] = fma(-l, prow[i], p[i]);
@@ -600,10 +674,20 @@ __device__ void bsolve(const T* W, int ld, int n, int k, Smem& sm, int my_pos, T
       load_row<T, NB>(W + (int64_t)(lane < nbj ? sm.piv[J + lane] : 0) * ld + J, nbj, uv);
       for_each_rhs(warp, k, [&](int c) {
         T y = lane < nbj ? (T)sm.vsm[lane][c] : T(0);
+        T rd = T(0), own = T(0);  // float: this lane's reciprocal, ahead of the chain
+        if constexpr (SHORT && sizeof(T) == 4) {
+#pragma unroll
+          for (int q = 0; q < NB; ++q)
+            if (q == lane) own = uv[q];
+          rd = brecip(own);
+        }
 #pragma unroll
         for (int q = NB - 1; q >= 0; --q) {
           if (q < nbj) {
-            if (lane == q) y = y / uv[q];
+            if (lane == q) {
+              if constexpr (SHORT && sizeof(T) == 4) y = rd != T(0) ? bquotient(y, own, rd) : bdivide_rare(y, own);
+              else y = y / uv[q];
+            }
             const T xq = __shfl_sync(0xffffffffu, y, q);
             if (lane < q) y = fma(-uv[q], xq, y);
           }
@@ -882,10 +966,20 @@ __device__ void bsolve_t(const T* W, int ld, int n, int k, Smem& sm, T (&v)[KMAX
         ucol[q] = (lane < nbj && q <= lane) ? W[(int64_t)sm.piv[J + q] * ld + J + lane] : T(0);
       for_each_rhs(warp, k, [&](int c) {
         T y = lane < nbj ? (T)sm.vsm[lane][c] : T(0);
+        T rd = T(0), own = T(0);  // float: this lane's reciprocal, ahead of the chain
+        if constexpr (sizeof(T) == 4) {
+#pragma unroll
+          for (int q = 0; q < NB; ++q)
+            if (q == lane) own = ucol[q];
+          rd = brecip(own);
+        }
 #pragma unroll
         for (int q = 0; q < NB; ++q) {
           if (q < nbj) {
-            if (lane == q) y = y / ucol[q];
+            if (lane == q) {
+              if constexpr (sizeof(T) == 4) y = rd != T(0) ? bquotient(y, own, rd) : bdivide_rare(y, own);
+              else y = y / ucol[q];
+            }
             const T zq = __shfl_sync(0xffffffffu, y, q);
             if (lane > q) y = fma(-ucol[q], zq, y);
           }
@@ -896,6 +990,7 @@ __device__ void bsolve_t(const T* W, int ld, int n, int k, Smem& sm, T (&v)[KMAX
     __syncthreads();
     if (t < n) {
       if (t >= J + nbj) {
+#pragma unroll 8
         for (int q = 0; q < nbj; ++q) {
           const T u = W[(int64_t)sm.piv[J + q] * ld + t];
 #pragma unroll
@@ -936,6 +1031,7 @@ __device__ void bsolve_t(const T* W, int ld, int n, int k, Smem& sm, T (&v)[KMAX
     __syncthreads();
     if (t < n) {
       if (t < J) {
+#pragma unroll 8
         for (int q = 0; q < nbj; ++q) {
           const T l = W[(int64_t)sm.piv[J + q] * ld + t];
 #pragma unroll
@@ -962,7 +1058,7 @@ __device__ double bresidual_t(const double* __restrict__ a, const double* __rest
     double acc[KMAX];
 #pragma unroll
     for (int c = 0; c < KMAX; ++c) acc[c] = 0.0;
-#pragma unroll 4
+#pragma unroll 8
     for (int i = 0; i < n; ++i) {
       const double av = __ldg(a + (int64_t)i * n + t);  // column t: coalesced across threads
       asum += fabs(av);
@@ -1101,11 +1197,16 @@ __global__ void __launch_bounds__(THREADS, RM_BT_MIN_BLOCKS) batch_adjoint_kerne
       for (int e = threadIdx.x; e < n * k; e += THREADS) sm.rs[e / k][e % k] = x[e];
       __syncthreads();
       double* ga = aj.ga + bt.a_off[s];
-      for (int e = threadIdx.x; e < n * n; e += THREADS) {
-        const int i = e / n, j = e - i * n;
-        double acc = 0.0;
-        for (int c = 0; c < k; ++c) acc = fma(sm.xs[i][c], sm.rs[j][c], acc);
-        ga[e] = -acc;
+      // a column per thread, the rows spread over the groups of threads left
+      const int width = (n + 31) & ~31, groups = THREADS / width;
+      const int grp = threadIdx.x / width, j = threadIdx.x - grp * width;
+      if (grp < groups && j < n) {
+#pragma unroll 4
+        for (int i = grp; i < n; i += groups) {
+          double acc = 0.0;
+          for (int c = 0; c < k; ++c) acc = fma(sm.xs[i][c], sm.rs[j][c], acc);
+          __stcs(ga + (int64_t)i * n + j, -acc);
+        }
       }
     }
     if (threadIdx.x == 0) aj.berr[s] = berr;
