@@ -63,6 +63,14 @@ __device__ __forceinline__ int exponent_of(double v) {
   return e;
 }
 
+// The largest finite magnitude first, then its exponent once: frexp an element costs more than
+// the pass over memory. A NaN never compares greater; an infinity (its exponent is not above that
+// of every finite entry) sends the caller through the entries one by one.
+__device__ __forceinline__ void max_magnitude(double& top, double v) {
+  v = fabs(v);
+  if (v > top) top = v;
+}
+
 // eb[j] (pre-set to INT_MIN) for each column of the k x n row-major b: 32 x 32 tiles, atomics
 __global__ void col_exponent_kernel(const double* __restrict__ b, int64_t ldb, int k, int n, int* __restrict__ eb) {
   __shared__ int cm[32];
@@ -70,9 +78,15 @@ __global__ void col_exponent_kernel(const double* __restrict__ b, int64_t ldb, i
   if (threadIdx.y == 0) cm[threadIdx.x] = INT_MIN;
   __syncthreads();
   int e = INT_MIN;
-  if (j < n)
-    for (int r = blockIdx.y * 32 + threadIdx.y; r < k; r += gridDim.y * 32)
-      e = max(e, exponent_of(fabs(b[(int64_t)r * ldb + j])));
+  if (j < n) {
+    const int r0 = blockIdx.y * 32 + threadIdx.y, step = gridDim.y * 32;
+    double top = 0.0;
+#pragma unroll 4
+    for (int r = r0; r < k; r += step) max_magnitude(top, b[(int64_t)r * ldb + j]);
+    e = exponent_of(top);
+    if (isinf(top))
+      for (int r = r0; r < k; r += step) e = max(e, exponent_of(fabs(b[(int64_t)r * ldb + j])));
+  }
   atomicMax(&cm[threadIdx.x], e);
   __syncthreads();
   if (threadIdx.y == 0 && j < n && cm[threadIdx.x] != INT_MIN) atomicMax(&eb[j], cm[threadIdx.x]);
@@ -86,49 +100,72 @@ __global__ void fix_exponent_kernel(int* e, int n) {
 // 2^e for -1022 <= e <= 1023
 __device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
 
-// The s signed base-128 digits of 2^-e x, truncated toward zero, the first in the low byte. For
-// a finite |2^-e x| < 1 they are those of one fixed-point number of 7 s bits, which costs one
-// conversion where a digit at a time costs two roundings each; the rest (a row or column with
-// an infinity) goes digit by digit.
-__device__ __forceinline__ uint64_t digits(double x, int e, int s) {
-  const double r = (unsigned)(e + 1022) <= 2044u ? x * pow2(-e) : ldexp(x, -e);
-  uint64_t out = 0;
-  if (fabs(r) < 1.0) {
-    uint64_t v = (uint64_t)__double2ll_rz(fabs(r) * pow2(7 * s));
-    const uint64_t neg = r < 0.0 ? 0xff : 0;
-    for (int p = s - 1; p >= 0; --p, v >>= 7) out |= ((((v & 127) ^ neg) - neg) & 0xff) << (8 * p);
-  } else {
-    double t = r;
-    for (int p = 0; p < s; ++p) {
-      t *= 128.0;
-      const double d = trunc(t);
-      t -= d;
-      out |= (uint64_t)(uint8_t)(int8_t)d << (8 * p);
-    }
-  }
-  return out;
+// Four bytes of 7 bits from 28 bits, the top ones in the high byte, each negated if neg
+__device__ __forceinline__ uint32_t spread7(uint32_t v, bool neg) {
+  v = (v & 0x3fffu) | ((v << 2) & 0x3fff0000u);
+  v = (v & 0x007f007fu) | ((v << 1) & 0x7f007f00u);
+  return neg ? (0x80808080u - v) ^ 0x80808080u : v;
 }
 
-// Byte p of four words of digits, the first word's lowest
-__device__ __forceinline__ uint32_t plane_word(const uint64_t (&w)[4], int p) {
-  const int sh = 8 * p;
-  return (uint32_t)((w[0] >> sh) & 0xff) | (uint32_t)((w[1] >> sh) & 0xff) << 8 |
-         (uint32_t)((w[2] >> sh) & 0xff) << 16 | (uint32_t)((w[3] >> sh) & 0xff) << 24;
+// The digits of a value that is not below 1 in magnitude (a row or column with an infinity, a
+// NaN), one by one
+__device__ __noinline__ uint2 digits_rare(double t) {
+  uint32_t w[2] = {0u, 0u};
+  for (int p = 0; p < MAX_SLICES; ++p) {
+    t *= 128.0;
+    const double d = trunc(t);
+    t -= d;
+    w[p >> 2] |= (uint32_t)(uint8_t)(int8_t)d << (8 * (3 - (p & 3)));
+  }
+  return make_uint2(w[0], w[1]);
+}
+
+// Eight signed base-128 digits of 2^-e x, truncated toward zero: x.x holds the first four, the
+// first in the high byte. They are the digits of one 56-bit fixed-point number, which costs one
+// conversion where a digit at a time costs two roundings each.
+__device__ __forceinline__ uint2 digits(double x, int e) {
+  const double r = (unsigned)(e + 1022) <= 2044u ? x * pow2(-e) : ldexp(x, -e);
+  if (!(fabs(r) < 1.0)) return digits_rare(r);
+  const uint64_t v = (uint64_t)__double2ll_rz(fabs(r) * 0x1p56);
+  return make_uint2(spread7((uint32_t)(v >> 28), r < 0.0), spread7((uint32_t)v & 0xfffffffu, r < 0.0));
+}
+
+// Words of planes 0..3 from the digit words of four elements: byte 3 - p of each, the first
+// element's lowest
+__device__ __forceinline__ void transpose4(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, uint32_t* out) {
+  const uint32_t a = __byte_perm(w0, w1, 0x6273), b = __byte_perm(w2, w3, 0x6273);  // planes 1 | 0
+  const uint32_t c = __byte_perm(w0, w1, 0x4051), d = __byte_perm(w2, w3, 0x4051);  // planes 3 | 2
+  out[0] = __byte_perm(a, b, 0x5410);
+  out[1] = __byte_perm(a, b, 0x7632);
+  out[2] = __byte_perm(c, d, 0x5410);
+  out[3] = __byte_perm(c, d, 0x7632);
+}
+__device__ __forceinline__ void plane_words(const double (&x)[4], int e, uint32_t (&out)[MAX_SLICES]) {
+  uint2 w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) w[i] = digits(x[i], e);
+  transpose4(w[0].x, w[1].x, w[2].x, w[3].x, out);
+  transpose4(w[0].y, w[1].y, w[2].y, w[3].y, out + 4);
 }
 
 // ea[i] and the s slices of row i of a into planes [p][i][kk] (row stride kp, plane stride
 // mp * kp), zero from k to kp: a block per row, so that the second pass over the row finds it
 // in L2, and four columns a lane, so that a warp's stores are 128 bytes in each plane. Rows
-// from m to mp stay unwritten: they only meet rows of C that are not stored.
+// from m to mp stay unwritten: they only meet rows of C that are not stored. HBM-bound but for the
+// second pass: 8192 x 8192, 198 us (157 for the bytes; with a digit at a time 421, and 410 : 244 for
+// the columns' kernel).
 __global__ void __launch_bounds__(256)
     split_rows_kernel(const double* __restrict__ a, int64_t lda, int k, int* __restrict__ ea, int s,
                       int8_t* __restrict__ out, int64_t kp, int64_t plane) {
   __shared__ int part[8];
   const int64_t row = blockIdx.x;
   const double* ar = a + row * lda;
-  int e = INT_MIN;
-#pragma unroll 4
-  for (int j = threadIdx.x; j < k; j += 256) e = max(e, exponent_of(fabs(ar[j])));
+  double top = 0.0;
+#pragma unroll 8
+  for (int j = threadIdx.x; j < k; j += 256) max_magnitude(top, ar[j]);
+  int e = exponent_of(top);
+  if (isinf(top))
+    for (int j = threadIdx.x; j < k; j += 256) e = max(e, exponent_of(fabs(ar[j])));
   e = __reduce_max_sync(0xffffffffu, e);
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = e;
   __syncthreads();
@@ -138,13 +175,13 @@ __global__ void __launch_bounds__(256)
   if (threadIdx.x == 0) ea[row] = e;
   for (int64_t j = 4 * threadIdx.x; j < kp; j += 1024) {
     double x[4];
-    uint64_t w[4];
+    uint32_t w[MAX_SLICES];
 #pragma unroll
     for (int i = 0; i < 4; ++i) x[i] = j + i < k ? ar[j + i] : 0.0;
+    plane_words(x, e, w);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) w[i] = digits(x[i], e, s);
-    for (int p = 0; p < s; ++p)
-      *reinterpret_cast<uint32_t*>(out + p * plane + row * kp + j) = plane_word(w, p);
+    for (int p = 0; p < MAX_SLICES; ++p)
+      if (p < s) *reinterpret_cast<uint32_t*>(out + p * plane + row * kp + j) = w[p];
   }
 }
 
@@ -163,15 +200,16 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
   for (int g = ty; g < 32; g += 8) {
     double x[4];
-    uint64_t w[4];
+    uint32_t w[MAX_SLICES];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int r = r0 + 4 * g + i;
       x[i] = (r < k && j < n) ? b[(int64_t)r * ldb + j] : 0.0;
     }
+    plane_words(x, e, w);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) w[i] = digits(x[i], e, s);
-    for (int q = 0; q < s; ++q) t8[q][tx][g] = plane_word(w, q);
+    for (int q = 0; q < MAX_SLICES; ++q)
+      if (q < s) t8[q][tx][g] = w[q];
   }
   __syncthreads();
   for (int i = ty; i < 32 * s; i += 8) {
@@ -214,7 +252,8 @@ __device__ __forceinline__ double scale_any(double v, int e) {
 // d - 1, so a loaded tile is used twice; with N = 256 that is 48 KB for 1024 cycles. Both
 // accumulators take all 512 TMEM columns, so the epilogue is not overlapped with the tile's
 // successor; it is under 3% of the 2d + 1 products, and C is read and written half as often.
-// 8192^3, 8 slices, the whole call: 22.7 ms before, 15.2 after.
+// 8192^3, 8 slices, the whole call: 22.7 ms before, 15.2 after, 14.9 with the split kernels above; the
+// tensor pipe then runs at 3.7 POPS (12.5 ms alone, 4.9 for the first launch) and the power cap binds.
 template <int BN, bool TWO>
 __global__ void __launch_bounds__(THREADS, 1)
     ozaki_order_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
