@@ -522,22 +522,61 @@ __global__ void __launch_bounds__(256) leaf_tail_kernel(double* w, int64_t ldw, 
   griddep_launch_dependents();
   griddep_wait();  // the kernel before this one in the stream has completed
   const LeafMoves& mv = s->moves[(j0 - J0) / kLeaf];
-  if (tid < kTailRows) from[tid] = -1;
-  for (int e = tid; e < kLeaf * kLeaf; e += 256) Lc[(e & 31) * kLeaf + (e >> 5)] = w[(int64_t)(j0 + (e >> 5)) * ldw + j0 + (e & 31)];
-  for (int e = tid; e < kTailRows * kLeaf; e += 256) {
-    const int r = e >> 5, q = e & 31;
-    A[r * kTailLda + q] = r0 + r < n ? -w[(int64_t)(r0 + r) * ldw + j0 + q] : 0.0;
+  if (warp == 0) {
+    const int disp = mv.disp, dst = mv.disp_dst[lane] - r0;
+    from[lane] = blockIdx.x == 0 ? lane : -1;
+    from[lane + kLeaf] = -1;
+    __syncwarp();
+    if (lane < disp && dst >= 0 && dst < kTailRows) from[dst] = kLeaf + lane;
   }
   double x[kLeaf];
   if (tid < cols)
 #pragma unroll
     for (int i = 0; i < kLeaf; ++i) x[i] = s->rows[i][off + tid];
-  __syncthreads();
-  if (tid < kLeaf) {
-    if (blockIdx.x == 0) from[tid] = tid;
-    const int d = tid < mv.disp ? mv.disp_dst[tid] - r0 : -1;
-    if (d >= 0 && d < kTailRows) from[d] = kLeaf + tid;
+  {
+    double lv[kLeaf / 8], av[kTailRows / 8];
+#pragma unroll
+    for (int i = 0; i < kLeaf / 8; ++i) lv[i] = w[(int64_t)(j0 + warp + 8 * i) * ldw + j0 + lane];
+#pragma unroll
+    for (int i = 0; i < kTailRows / 8; ++i) {
+      const int r = r0 + warp + 8 * i;
+      av[i] = r < n ? -w[(int64_t)r * ldw + j0 + lane] : 0.0;
+    }
+#pragma unroll
+    for (int i = 0; i < kLeaf / 8; ++i) Lc[lane * kLeaf + warp + 8 * i] = lv[i];
+#pragma unroll
+    for (int i = 0; i < kTailRows / 8; ++i) A[(warp + 8 * i) * kTailLda + lane] = av[i];
   }
+  __syncthreads();
+  // The update's rows and the moved rows' columns left of the leaf (at most 64) are asked for here, to
+  // arrive behind U12: loaded one after another where they are used, they were most of this kernel.
+  const int g = lane >> 2, q = lane & 3, m0 = 16 * (warp >> 1);
+  const bool update = blockIdx.x != 0 || m0 >= kLeaf;  // not the diagonal rows
+  const int ra = m0 + g, rb = ra + 8;
+  const bool va = update && r0 + ra < n, vb = update && r0 + rb < n;
+  double acc[6][4];
+  {
+    const double* srca = from[ra] >= 0 ? s->rows[from[ra]] + off : w + (int64_t)(r0 + ra) * ldw + c0;
+    const double* srcb = from[rb] >= 0 ? s->rows[from[rb]] + off : w + (int64_t)(r0 + rb) * ldw + c0;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+      const int c = 48 * (warp & 1) + 8 * j + 2 * q;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        acc[j][h] = va && c + h < cols ? srca[c + h] : 0.0;
+        acc[j][2 + h] = vb && c + h < cols ? srcb[c + h] : 0.0;
+      }
+    }
+  }
+  constexpr int kLeft = (kOuter - 2 * kLeaf) / 32;
+  double moved[kTailRows / 8][kLeft];
+#pragma unroll
+  for (int i = 0; i < kTailRows / 8; ++i)
+#pragma unroll
+    for (int h = 0; h < kLeft; ++h) {
+      const int e = from[warp + 8 * i], c = lane + 32 * h;
+      moved[i][h] = e >= 0 && c < j0 - J0 ? s->rows[e][c] : 0.0;
+    }
   if (tid < cols) {
 #pragma unroll
     for (int i = 0; i < kLeaf - 1; ++i) {
@@ -552,28 +591,14 @@ __global__ void __launch_bounds__(256) leaf_tail_kernel(double* w, int64_t ldw, 
       for (int i = 0; i < kLeaf; ++i) w[(int64_t)(j0 + i) * ldw + c0 + tid] = x[i];
   }
   __syncthreads();
-  // the moved rows' columns left of the leaf
-  for (int r = warp; r < kTailRows; r += 8) {
-    const int e = from[r];
-    if (e >= 0)
-      for (int c = lane; c < j0 - J0; c += 32) w[(int64_t)(r0 + r) * ldw + J0 + c] = s->rows[e][c];
-  }
-  const int g = lane >> 2, q = lane & 3, m0 = 16 * (warp >> 1);
-  if (blockIdx.x == 0 && m0 < kLeaf) return;  // the diagonal rows
-  const int ra = m0 + g, rb = ra + 8;
-  const double* srca = from[ra] >= 0 ? s->rows[from[ra]] + off : w + (int64_t)(r0 + ra) * ldw + c0;
-  const double* srcb = from[rb] >= 0 ? s->rows[from[rb]] + off : w + (int64_t)(r0 + rb) * ldw + c0;
-  const bool va = r0 + ra < n, vb = r0 + rb < n;
-  double acc[6][4];
 #pragma unroll
-  for (int j = 0; j < 6; ++j) {
-    const int c = 48 * (warp & 1) + 8 * j + 2 * q;
+  for (int i = 0; i < kTailRows / 8; ++i)
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      acc[j][h] = va && c + h < cols ? srca[c + h] : 0.0;
-      acc[j][2 + h] = vb && c + h < cols ? srcb[c + h] : 0.0;
+    for (int h = 0; h < kLeft; ++h) {
+      const int r = warp + 8 * i, c = lane + 32 * h;
+      if (from[r] >= 0 && c < j0 - J0) w[(int64_t)(r0 + r) * ldw + J0 + c] = moved[i][h];
     }
-  }
+  if (!update) return;
 #pragma unroll
   for (int k = 0; k < kLeaf; k += 8) {
     const double a[4] = {A[ra * kTailLda + k + q], A[rb * kTailLda + k + q], A[ra * kTailLda + k + q + 4],
@@ -607,13 +632,17 @@ int leaf_tail_f64(double* w, int64_t ldw, int n, int j0, int J0, int J1, const B
 // A CTA per 64 columns outside the block (all of those left of it, or none, and lo .. hi - 1 of
 // those right of it): the net moves of the block's four leaves, then, right of the block, U12 =
 // L11^-1 A12 in shared memory: the four 32 x 32 diagonal blocks of L11 are inverted by a warp each
-// (a lane per column) while the other warps fetch the rows, and per block row X_b = D_b^-1 (A_b -
+// (a lane per column) while the other warps work out the moves, and per block row X_b = D_b^-1 (A_b -
 // sum) and the rows below it are updated, all on DMMA. One launch in place of a swap, an inversion
 // of the whole L11 and a product with it. 64 columns: the lists, L11 and its inverses are per CTA,
 // and at 8192 columns the CTAs still fit one wave.
 constexpr int kBrCols = 64;
 constexpr int kBrLdx = kBrCols + 4;   // fragment loads of both operands hit 16 distinct 8-byte banks
 constexpr int kBrLda = kOuter + 4;
+// where the inverse of L11's diagonal block b lies: blocks (0, 1), (1, 2), (2, 3) and (0, 3)
+__device__ __forceinline__ int inverse_at(int b) {
+  return b < kOuter / kLeaf - 1 ? kLeaf * b * kBrLda + kLeaf * (b + 1) : kLeaf * b;
+}
 constexpr size_t kBrSmem = ((size_t)kOuter * kBrLdx + (size_t)kOuter * kBrLda) * sizeof(double);
 
 __global__ void __launch_bounds__(256) block_rows_kernel(double* w, int64_t ldw, int J0, int nb, int left_cols, int lo,
@@ -622,6 +651,7 @@ __global__ void __launch_bounds__(256) block_rows_kernel(double* w, int64_t ldw,
   double* X = bsm;                      // [128][kBrLdx]: the block's rows
   double* L = bsm + kOuter * kBrLdx;    // [128][kBrLda]: L11, D_b^-1 in its diagonal blocks
   __shared__ LeafMoves mv[kOuter / kLeaf];
+  __shared__ int4 dsts[kOuter / kLeaf][kLeaf / 4];  // disp_dst, -1 past disp
   __shared__ int src[kOuter], xdst[kOuter], xsrc[kOuter], extra;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int leaves = (nb + kLeaf - 1) / kLeaf, J1 = J0 + nb;
@@ -641,8 +671,26 @@ __global__ void __launch_bounds__(256) block_rows_kernel(double* w, int64_t ldw,
   }
   for (int e = tid; e < leaves * (int)(sizeof(LeafMoves) / 4); e += 256)
     reinterpret_cast<int*>(mv)[e] = reinterpret_cast<const int*>(s->moves)[e];
+  if (tid < kOuter) {
+    const int l = tid / kLeaf, d = tid % kLeaf;
+    reinterpret_cast<int*>(dsts)[tid] = l < leaves && d < s->moves[l].disp ? s->moves[l].disp_dst[d] : -1;
+  }
   if (tid == 0) extra = 0;
+  cp_async_wait_all();
   __syncthreads();
+  // the displaced row of leaf l that ends at position p, or -1
+  auto find = [&](int p, int l) {
+    int at = -1;
+#pragma unroll
+    for (int i = 0; i < kLeaf / 4; ++i) {
+      const int4 v = dsts[l][i];
+      if (v.x == p) at = 4 * i;
+      if (v.y == p) at = 4 * i + 1;
+      if (v.z == p) at = 4 * i + 2;
+      if (v.w == p) at = 4 * i + 3;
+    }
+    return at;
+  };
   // the row that ends at position p after all leaves was at position back(p, leaves) before them
   auto back = [&](int p, int l) {
     for (--l; l >= 0; --l) {
@@ -650,26 +698,36 @@ __global__ void __launch_bounds__(256) block_rows_kernel(double* w, int64_t ldw,
       if (p >= m.j0 && p < m.j0 + m.jb) {
         p = m.piv_src[p - m.j0];
       } else {
-        int found = p;
-#pragma unroll 8
-        for (int d = 0; d < kLeaf; ++d)
-          if (d < m.disp && m.disp_dst[d] == p) found = m.disp_src[d];
-        p = found;
+        const int d = find(p, l);
+        if (d >= 0) p = m.disp_src[d];
       }
     }
     return p;
   };
-  if (tid < kOuter) {
-    src[tid] = tid < nb ? back(J0 + tid, leaves) : J0 + tid;
-  } else {
+  const bool invert_ahead = solve && cols > 0;
+  const int lt = invert_ahead ? tid - kOuter : tid;  // the lists by warps 4..7 beside the inverses, or by all
+  if (invert_ahead && warp < 4) {
+    // D_b^-1 of the diagonal block b = warp, a lane per column, into a block of L's unused upper part
+    const double* D = L + (kLeaf * warp) * kBrLda + kLeaf * warp;
+    double x[kLeaf];
+#pragma unroll
+    for (int i = 0; i < kLeaf; ++i) x[i] = i == lane ? 1.0 : 0.0;
+#pragma unroll
+    for (int i = 0; i < kLeaf - 1; ++i)
+#pragma unroll
+      for (int r = i + 1; r < kLeaf; ++r) x[r] = fma(D[r * kBrLda + i], -x[i], x[r]);
+    double* V = L + inverse_at(warp);
+#pragma unroll
+    for (int i = 0; i < kLeaf; ++i) V[i * kBrLda + lane] = x[i];
+  }
+  if (lt >= 0 && lt < kOuter) src[lt] = lt < nb ? back(J0 + lt, leaves) : J0 + lt;
+  if (tid >= kOuter) {
     // positions below the block, each once: by the last leaf that moved a row there
     const int l = (tid - kOuter) / kLeaf, d = (tid - kOuter) % kLeaf;
     if (l < leaves && d < mv[l].disp && mv[l].disp_dst[d] >= J1) {
       const int p = mv[l].disp_dst[d];
       bool last = true;
-      for (int l2 = l + 1; l2 < leaves; ++l2)
-#pragma unroll 8
-        for (int d2 = 0; d2 < kLeaf; ++d2) last &= d2 >= mv[l2].disp || mv[l2].disp_dst[d2] != p;
+      for (int l2 = l + 1; l2 < leaves; ++l2) last &= find(p, l2) < 0;
       const int from = last ? back(p, leaves) : p;
       if (last && from != p) {
         const int e = atomicAdd(&extra, 1);
@@ -678,7 +736,6 @@ __global__ void __launch_bounds__(256) block_rows_kernel(double* w, int64_t ldw,
       }
     }
   }
-  cp_async_wait_all();
   __syncthreads();
   const int extras = extra;
   if (perm != nullptr && blockIdx.x == 0) {
@@ -728,20 +785,6 @@ __global__ void __launch_bounds__(256) block_rows_kernel(double* w, int64_t ldw,
       for (int i = 1; i < kOuter; ++i)
         for (int r = 0; r < i; ++r) X[i * kBrLdx + tid] = fma(L[i * kBrLda + r], -X[r * kBrLdx + tid], X[i * kBrLdx + tid]);
   }
-  if (invert && warp < 4) {
-    // D_b^-1 of the diagonal block b = warp, a lane per column, in place
-    double* D = L + (kLeaf * warp) * kBrLda + kLeaf * warp;
-    double x[kLeaf];
-#pragma unroll
-    for (int i = 0; i < kLeaf; ++i) x[i] = i == lane ? 1.0 : 0.0;
-#pragma unroll
-    for (int i = 0; i < kLeaf - 1; ++i)
-#pragma unroll
-      for (int r = i + 1; r < kLeaf; ++r) x[r] = fma(D[r * kBrLda + i], -x[i], x[r]);
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < kLeaf; ++i) D[i * kBrLda + lane] = x[i];
-  }
   __syncthreads();
 #pragma unroll
   for (int q = 0; q < kOuter / 8; ++q) {
@@ -757,7 +800,7 @@ __global__ void __launch_bounds__(256) block_rows_kernel(double* w, int64_t ldw,
       double d[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
 #pragma unroll
       for (int k = 0; k < kLeaf; k += 8) {
-        const double* a0 = L + (m0 + g) * kBrLda + kLeaf * b + k + q;
+        const double* a0 = L + inverse_at(b) + (16 * (warp >> 2) + g) * kBrLda + k + q;
         const double a[4] = {a0[0], a0[8 * kBrLda], a0[4], a0[8 * kBrLda + 4]};
         const double* x0 = X + (kLeaf * b + k + q) * kBrLdx + n0 + g;
         dmma(d[0], a, x0[0], x0[4 * kBrLdx]);
