@@ -149,11 +149,11 @@ static int finish_call(cudaStream_t s, const int32_t* d_flag, int32_t* flag, con
 // ------------------------------------------------------------------ failure injection (tests)
 // Per thread and RM_INJECT_* kind: how many events pass before the next failures, and how
 // many fail then.
-static thread_local int g_inject_after[3] = {0, 0, 0};
-static thread_local int g_inject_count[3] = {0, 0, 0};
+static thread_local int g_inject_after[RM_INJECT_KINDS + 1] = {};
+static thread_local int g_inject_count[RM_INJECT_KINDS + 1] = {};
 
 bool injected_failure(int kind) {
-  if (kind < 1 || kind > 2 || g_inject_count[kind] <= 0) return false;
+  if (kind < 1 || kind > RM_INJECT_KINDS || g_inject_count[kind] <= 0) return false;
   if (g_inject_after[kind] > 0) {
     --g_inject_after[kind];
     return false;
@@ -369,7 +369,7 @@ int rm_take_status(void* stream) {
 }
 
 int rm_test_inject_failure(int kind, int after, int count) {
-  if (kind < 1 || kind > 2 || after < 0 || count < 0) return RM_BAD_ARG;
+  if (kind < 1 || kind > RM_INJECT_KINDS || after < 0 || count < 0) return RM_BAD_ARG;
   g_inject_after[kind] = after;
   g_inject_count[kind] = count;
   return RM_OK;

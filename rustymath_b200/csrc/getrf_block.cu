@@ -78,6 +78,10 @@ struct LeafShared {
   alignas(16) double piv_other[kLeaf][kOuter];
   alignas(16) double top_other[kLeaf][kOuter];
 };
+// the self-test's column whose posts come short, and its waits' limit
+constexpr int kHoldColumn = 11;
+constexpr uint64_t kSelfTestWaitNs = 1000000;
+
 constexpr size_t leaf_smem(int threads) {
   return (sizeof(LeafShared) + 15) / 16 * 16 + (size_t)threads * kLeafStride * sizeof(double);
 }
@@ -114,7 +118,7 @@ __device__ __forceinline__ int leaf_best(unsigned hi, unsigned lo, unsigned pos)
 template <bool CLUSTER>
 __global__ void __launch_bounds__(kLeafMaxThreads, 1)
     leaf_kernel(double* w, int64_t ldw, int n, int j0, int jb, int J0, int J1, BlockScratch* s, LeafMarks* marks,
-                unsigned* status) {
+                unsigned* status, uint64_t wait_ns, bool hold) {
   extern __shared__ __align__(16) uint8_t smem[];
   LeafShared& sh = *reinterpret_cast<LeafShared*>(smem);
   double* S = reinterpret_cast<double*>(smem + (sizeof(LeafShared) + 15) / 16 * 16);
@@ -133,11 +137,19 @@ __global__ void __launch_bounds__(kLeafMaxThreads, 1)
       mbar_init(&sh.bar[t], 1);
       if (t < kLeaf / kSub) mbar_init(&sh.row_bar[t], 1);
       fence_barrier_init();
-      mbar_arrive_expect_tx(&sh.bar[t], (uint32_t)C * sizeof(LeafPost));
+      const uint32_t held = hold && t == kHoldColumn ? 16u : 0u;  // bytes that nobody sends
+      mbar_arrive_expect_tx(&sh.bar[t], (uint32_t)C * sizeof(LeafPost) + held);
       if (t < kLeaf / kSub) mbar_arrive_expect_tx(&sh.row_bar[t], kSub * (kLeaf - kSub * t) * 8);
     }
   }
   griddep_wait();  // the kernel before this one in the stream has completed
+  // A list that moves nothing, for the launches behind this one should a wait give up before the moves
+  // are known; each CTA's own part of the list replaces it at the end, behind a cluster barrier.
+  if (CLUSTER && rank == 0 && t < jb) {
+    LeafMoves& mv = s->moves[(j0 - J0) / kLeaf];
+    mv.piv_src[t] = j0 + t;
+    if (t == 0) mv.j0 = j0, mv.jb = jb, mv.disp = 0;
+  }
   // the rows into shared memory: 16 lanes per row (coalesced), then a row per thread
   const double* g = w + (int64_t)(j0 + r0) * ldw + j0;
   for (int e = t; e < rows * (kLeaf / 2); e += T) {
@@ -161,10 +173,14 @@ __global__ void __launch_bounds__(kLeafMaxThreads, 1)
   // where this warp sends its CTA's posts: CTA `warp` (and warp + warps, ... of a wide cluster)
   const uint32_t rpost = CLUSTER ? map_rank(&sh.cta_post[0][rank], min(warp, C - 1)) + lane * 16u : 0u;
   const uint32_t rbar = CLUSTER ? map_rank(&sh.bar[0], min(warp, C - 1)) : 0u;
-  // a wait gave up: leave once no copy of this CTA's is in flight and no CTA sends to it any more
+  // a wait gave up: leave once no copy of this CTA's is in flight, no CTA sends to it any more, and
+  // what was sent to it before (microseconds at most) has landed
   auto give_up = [] {
+    __syncwarp();
     cp_async_wait<0>();
     cluster_sync_all();
+    for (const uint64_t start = global_ns(); global_ns() - start < 20000;) {
+    }
   };
   double* srow = S + t * kLeafStride;
   bool active = t < rows;
@@ -208,7 +224,7 @@ __global__ void __launch_bounds__(kLeafMaxThreads, 1)
           for (int dst = warp + warps; dst < C; dst += warps)
             st_async16(map_rank(&sh.cta_post[i & 1][rank], dst) + lane * 16u, v, map_rank(&sh.bar[c], dst));
         }
-        if (!mbar_wait_cluster(&sh.bar[c], 0, status)) return give_up();
+        if (!mbar_wait_cluster(&sh.bar[c], 0, status, wait_ns)) return give_up();
         const LeafPost* cp = sh.cta_post[i & 1];
         m = lane < C ? *reinterpret_cast<const uint4*>(&cp[lane].hi) : make_uint4(0u, 0u, kNone, 0u);
         win = &cp[leaf_best(m.x, m.y, m.z)];
@@ -268,7 +284,7 @@ __global__ void __launch_bounds__(kLeafMaxThreads, 1)
     const int rc0 = c0 + kSub;
     if (rc0 >= jb) break;
     if (CLUSTER) {
-      if (!mbar_wait_cluster(&sh.row_bar[c0 / kSub], 0, status)) return give_up();
+      if (!mbar_wait_cluster(&sh.row_bar[c0 / kSub], 0, status, wait_ns)) return give_up();
     } else {
       __syncthreads();
     }
@@ -399,7 +415,7 @@ int leaf_f64(double* w, int64_t ldw, int n, int j0, int jb, int J0, int J1, Bloc
   if (C == 1) {
     RM_TRY(smem_attribute(leaf_kernel<false>, leaf_smem(kLeafMaxThreads)));
     RM_CUDA_TRY(launch_dependent(leaf_kernel<false>, dim3(1), dim3(T), leaf_smem(T), stream, w, ldw, n, j0, jb, J0, J1, s,
-                                 marks, status));
+                                 marks, status, kWaitLimitNs, false));
     note_launch();
     return RM_OK;
   }
@@ -418,7 +434,9 @@ int leaf_f64(double* w, int64_t ldw, int n, int j0, int jb, int J0, int J1, Bloc
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  RM_CUDA_TRY(cudaLaunchKernelEx(&cfg, leaf_kernel<true>, w, ldw, n, j0, jb, J0, J1, s, marks, status));
+  const bool hold = injected_failure(RM_INJECT_LEAF_TIMEOUT);  // a self-test's leaf
+  RM_CUDA_TRY(cudaLaunchKernelEx(&cfg, leaf_kernel<true>, w, ldw, n, j0, jb, J0, J1, s, marks, status,
+                                 hold ? kSelfTestWaitNs : kWaitLimitNs, hold));
   note_launch();
   return RM_OK;
 }

@@ -49,8 +49,8 @@ __device__ __forceinline__ void st_async16(uint32_t dst, double2 v, uint32_t bar
                : "memory");
 }
 
-// mbar_wait for a barrier that other CTAs' st_async16 complete on.
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, unsigned* status) {
+// mbar_wait, with a limit of its own, for a barrier that other CTAs' st_async16 complete on.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, unsigned* status, uint64_t wait_ns) {
   const uint32_t a = smem_u32(bar);
   uint64_t start = 0;
   for (int i = 0;; ++i) {
@@ -65,7 +65,7 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
     if ((i & 63) == 63) {
       const uint64_t now = global_ns();
       if (!start) start = now;
-      else if (now - start > kWaitLimitNs) break;
+      else if (now - start > wait_ns) break;
     }
   }
   flag_error(status, RM_DEV_TIMEOUT);
