@@ -95,10 +95,11 @@ int rm_take_status(void *stream);
  * hangs because of them. */
 #define RM_INJECT_OUT_OF_MEMORY 1 /* a scratch allocation reports device memory exhausted */
 #define RM_INJECT_CUDA_ERROR 2    /* a scratch allocation fails with a CUDA error */
-/* The CTAs of a float64 LU leaf wait for a post that does not come: the waits give up after 1 ms and
- * the factorization reports RM_TIMEOUT. */
+/* A float64 LU leaf of more than one CTA waits for posts that do not come, in all of its CTAs or in
+ * the last one only: its waits give up after 1 ms and the factorization reports RM_TIMEOUT. */
 #define RM_INJECT_LEAF_TIMEOUT 3
-#define RM_INJECT_KINDS 3
+#define RM_INJECT_LEAF_CTA_TIMEOUT 4
+#define RM_INJECT_KINDS 4
 /* On the calling thread, after the next `after` events of `kind` succeed, `count` more fail
  * as described; count 0 disarms. */
 int rm_test_inject_failure(int kind, int after, int count);

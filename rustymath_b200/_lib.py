@@ -12,7 +12,7 @@ RM_OK, RM_BAD_ARG, RM_NOT_REGULAR, RM_CUDA_ERROR = 0, 1, 2, 3
 RM_TIMEOUT, RM_NO_CONVERGENCE, RM_NO_DEVICE, RM_OUT_OF_MEMORY = 4, 5, 6, 7
 RM_NOT_POSITIVE_DEFINITE = 8
 RM_METHOD_PLAIN_F64, RM_METHOD_F32_IR, RM_METHOD_GMRES_IR = 0, 1, 2
-RM_INJECT_OUT_OF_MEMORY, RM_INJECT_CUDA_ERROR, RM_INJECT_LEAF_TIMEOUT = 1, 2, 3
+RM_INJECT_OUT_OF_MEMORY, RM_INJECT_CUDA_ERROR, RM_INJECT_LEAF_TIMEOUT, RM_INJECT_LEAF_CTA_TIMEOUT = 1, 2, 3, 4
 
 _i32, _i64, _f64, _p = ctypes.c_int32, ctypes.c_int64, ctypes.c_double, ctypes.c_void_p
 

@@ -78,7 +78,7 @@ struct LeafShared {
   alignas(16) double piv_other[kLeaf][kOuter];
   alignas(16) double top_other[kLeaf][kOuter];
 };
-// the self-test's column whose posts come short, and its waits' limit
+// the self-test's column whose posts come short (in the CTAs of `hold`)
 constexpr int kHoldColumn = 11;
 constexpr uint64_t kSelfTestWaitNs = 1000000;
 
@@ -118,7 +118,7 @@ __device__ __forceinline__ int leaf_best(unsigned hi, unsigned lo, unsigned pos)
 template <bool CLUSTER>
 __global__ void __launch_bounds__(kLeafMaxThreads, 1)
     leaf_kernel(double* w, int64_t ldw, int n, int j0, int jb, int J0, int J1, BlockScratch* s, LeafMarks* marks,
-                unsigned* status, uint64_t wait_ns, bool hold) {
+                unsigned* status, uint64_t wait_ns, unsigned hold) {
   extern __shared__ __align__(16) uint8_t smem[];
   LeafShared& sh = *reinterpret_cast<LeafShared*>(smem);
   double* S = reinterpret_cast<double*>(smem + (sizeof(LeafShared) + 15) / 16 * 16);
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(kLeafMaxThreads, 1)
       mbar_init(&sh.bar[t], 1);
       if (t < kLeaf / kSub) mbar_init(&sh.row_bar[t], 1);
       fence_barrier_init();
-      const uint32_t held = hold && t == kHoldColumn ? 16u : 0u;  // bytes that nobody sends
+      const uint32_t held = t == kHoldColumn && ((hold >> rank) & 1u) ? 16u : 0u;  // bytes that nobody sends
       mbar_arrive_expect_tx(&sh.bar[t], (uint32_t)C * sizeof(LeafPost) + held);
       if (t < kLeaf / kSub) mbar_arrive_expect_tx(&sh.row_bar[t], kSub * (kLeaf - kSub * t) * 8);
     }
@@ -173,10 +173,13 @@ __global__ void __launch_bounds__(kLeafMaxThreads, 1)
   // where this warp sends its CTA's posts: CTA `warp` (and warp + warps, ... of a wide cluster)
   const uint32_t rpost = CLUSTER ? map_rank(&sh.cta_post[0][rank], min(warp, C - 1)) + lane * 16u : 0u;
   const uint32_t rbar = CLUSTER ? map_rank(&sh.bar[0], min(warp, C - 1)) : 0u;
-  // a wait gave up: leave once no copy of this CTA's is in flight, no CTA sends to it any more, and
+  // Whether this thread's waits have all ended in time. A thread whose wait gave up stays in step (the
+  // others may have seen the same posts arrive, and count on it at the CTA's barriers) but sends no
+  // post, waits for none and takes no position from one; the CTA agrees at the sub-leaf's barriers.
+  bool ok = true;
+  // the CTA leaves together: once no copy of its own is in flight, no CTA sends to it any more, and
   // what was sent to it before (microseconds at most) has landed
   auto give_up = [] {
-    __syncwarp();
     cp_async_wait<0>();
     cluster_sync_all();
     for (const uint64_t start = global_ns(); global_ns() - start < 20000;) {
@@ -218,13 +221,14 @@ __global__ void __launch_bounds__(kLeafMaxThreads, 1)
       uint4 m = lane < warps ? *reinterpret_cast<const uint4*>(&wp[lane].hi) : make_uint4(0u, 0u, kNone, 0u);
       const LeafPost* win = &wp[leaf_best(m.x, m.y, m.z)];
       if (CLUSTER) {
-        if (warp < C && lane < kPostPieces) {
+        if (ok && warp < C && lane < kPostPieces) {
           const double2 v = reinterpret_cast<const double2*>(win)[lane];
           st_async16(rpost + (i & 1) * (uint32_t)sizeof(sh.cta_post[0]), v, rbar + c * 8u);
           for (int dst = warp + warps; dst < C; dst += warps)
             st_async16(map_rank(&sh.cta_post[i & 1][rank], dst) + lane * 16u, v, map_rank(&sh.bar[c], dst));
         }
-        if (!mbar_wait_cluster(&sh.bar[c], 0, status, wait_ns)) return give_up();
+        ok = ok && mbar_wait_cluster(&sh.bar[c], 0, status, wait_ns);
+        __syncwarp();
         const LeafPost* cp = sh.cta_post[i & 1];
         m = lane < C ? *reinterpret_cast<const uint4*>(&cp[lane].hi) : make_uint4(0u, 0u, kNone, 0u);
         win = &cp[leaf_best(m.x, m.y, m.z)];
@@ -235,12 +239,14 @@ __global__ void __launch_bounds__(kLeafMaxThreads, 1)
       double2 u[kSub / 2];
 #pragma unroll
       for (int q = i / 2; q < kSub / 2; ++q) u[q] = reinterpret_cast<const double2*>(win->row)[q];
-      if (pos == (int)meta.x) {
-        active = false;
-        pos = c;
-        sh.chosen[c] = t;
-      } else if (pos == c) {
-        pos = (int)meta.x;
+      if (ok) {
+        if (pos == (int)meta.x) {
+          active = false;
+          pos = c;
+          sh.chosen[c] = t;
+        } else if (pos == c) {
+          pos = (int)meta.x;
+        }
       }
       double l = p[i] * r;
       if (meta.y != kPivotInvert) {
@@ -261,7 +267,11 @@ __global__ void __launch_bounds__(kLeafMaxThreads, 1)
       for (int i = 0; i < kSub; i += 2) *reinterpret_cast<double2*>(srow + c0 + i) = make_double2(p[i], p[i + 1]);
     }
     sh.active[t] = active;
-    __syncthreads();
+    if (CLUSTER) {
+      if (!__syncthreads_and(ok)) return give_up();
+    } else {
+      __syncthreads();
+    }
     // the pivot rows held here: their other columns of the block in the background; to every CTA,
     // the row from the sub-leaf's columns on
     for (int k = warp; k < kSub; k += warps) {
@@ -284,7 +294,8 @@ __global__ void __launch_bounds__(kLeafMaxThreads, 1)
     const int rc0 = c0 + kSub;
     if (rc0 >= jb) break;
     if (CLUSTER) {
-      if (!mbar_wait_cluster(&sh.row_bar[c0 / kSub], 0, status, wait_ns)) return give_up();
+      ok = mbar_wait_cluster(&sh.row_bar[c0 / kSub], 0, status, wait_ns);
+      __syncwarp();
     } else {
       __syncthreads();
     }
@@ -312,7 +323,11 @@ __global__ void __launch_bounds__(kLeafMaxThreads, 1)
         sh.prow[k][col] = ((skip >> k) & 1u) ? 0.0 : u[k];
       }
     }
-    __syncthreads();
+    if (CLUSTER) {
+      if (!__syncthreads_and(ok)) return give_up();
+    } else {
+      __syncthreads();
+    }
     // the rows not yet chosen: later columns -= L U12, an m16 tile of rows per warp at a time
     {
       const int g2 = lane >> 2, q = lane & 3;
@@ -415,7 +430,7 @@ int leaf_f64(double* w, int64_t ldw, int n, int j0, int jb, int J0, int J1, Bloc
   if (C == 1) {
     RM_TRY(smem_attribute(leaf_kernel<false>, leaf_smem(kLeafMaxThreads)));
     RM_CUDA_TRY(launch_dependent(leaf_kernel<false>, dim3(1), dim3(T), leaf_smem(T), stream, w, ldw, n, j0, jb, J0, J1, s,
-                                 marks, status, kWaitLimitNs, false));
+                                 marks, status, kWaitLimitNs, 0u));
     note_launch();
     return RM_OK;
   }
@@ -434,7 +449,9 @@ int leaf_f64(double* w, int64_t ldw, int n, int j0, int jb, int J0, int J1, Bloc
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const bool hold = injected_failure(RM_INJECT_LEAF_TIMEOUT);  // a self-test's leaf
+  unsigned hold = 0u;  // a self-test's leaf, with a short limit
+  if (injected_failure(RM_INJECT_LEAF_TIMEOUT)) hold = 0xffffffffu;
+  else if (injected_failure(RM_INJECT_LEAF_CTA_TIMEOUT)) hold = 1u << (C - 1);
   RM_CUDA_TRY(cudaLaunchKernelEx(&cfg, leaf_kernel<true>, w, ldw, n, j0, jb, J0, J1, s, marks, status,
                                  hold ? kSelfTestWaitNs : kWaitLimitNs, hold));
   note_launch();
