@@ -87,17 +87,13 @@ constexpr size_t leaf_smem(int threads) {
 }
 static_assert(leaf_smem(kLeafMaxThreads) <= 227 * 1024, "a CTA's shared memory");
 
-// 1 / a from the hardware's approximation x0 (20 bits): e = 1 - a x0, x = x0 (1 + e + e^2), which
-// leaves e^3, then one Newton step to round. No branches, so that it runs beside the reduction. 0
-// where the pivot is divided by instead: subnormal or too large to invert.
-__device__ __forceinline__ double leaf_rcp(double a) {
-  double x0;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x0) : "d"(a));
-  const double e = fma(-a, x0, 1.0);
-  double x = fma(x0, fma(e, e, e), x0);
-  x = fma(x, fma(-a, x, 1.0), x);
-  const bool sub = ((unsigned)__double2hiint(a) & 0x7ff00000u) == 0u, flushed = (__double2hiint(x0) & 0x7fffffff) == 0;
-  return sub || flushed ? 0.0 : x;
+// 1 / a, correctly rounded; 0 where rustymath divides by the pivot instead (a subnormal one). Every lane
+// forms its own beside the reduction. Rows that are no candidates give 1 to the intrinsic, so that it
+// leaves its short path for extreme pivots only.
+__device__ __forceinline__ double leaf_rcp(double a, bool candidate) {
+  const bool normal = ((unsigned)__double2hiint(a) & 0x7ff00000u) != 0u;
+  const double r = __drcp_rn(candidate && normal ? a : 1.0);
+  return normal ? r : 0.0;
 }
 
 // A candidate's key: the bits of its magnitude, the high word plus 2. 0: no candidate; 1: a NaN at
@@ -207,7 +203,7 @@ __global__ void __launch_bounds__(kLeafMaxThreads, 1)
       unsigned hi = 0u;
       if (active) hi = mag <= 0x7ff0000000000000ull ? (unsigned)(mag >> 32) + 2u : (pos == c ? 1u : 0u);
       const unsigned lo = (unsigned)mag;
-      const double rcp = leaf_rcp(p[i]);
+      const double rcp = leaf_rcp(p[i], active);
       LeafPost* wp = sh.warp_post[i & 1];
       if (lane == leaf_best(hi, lo, (unsigned)pos)) {
         LeafPost& post = wp[warp];
