@@ -34,8 +34,6 @@
 // that kernel's end; it reads nothing of it before griddepcontrol.wait).
 #include <climits>
 
-#include <cfloat>
-
 #include "rm_internal.h"
 
 namespace rm {
@@ -82,16 +80,6 @@ static_assert(kLppThreads == 256, "the pivot search reduces 8 warp posts");
 __device__ __forceinline__ unsigned pivot_key(float v) {
   const float a = fabsf(v);
   return a != a ? 1u : __float_as_uint(a) + 2u;
-}
-
-// 1 / a from the hardware's approximation and one Newton step x += x (1 - a x), within an ulp. The
-// correctly rounded sequence branches and takes ~130 cycles, on the path of every column; this runs
-// beside the reduction. Where the step is not finite the approximation stands (0 for an infinity).
-__device__ __forceinline__ float lpp_rcp(float a) {
-  float x;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(x) : "f"(a));
-  const float y = fmaf(x, fmaf(-a, x, 1.0f), x);
-  return fabsf(y) <= FLT_MAX ? y : x;
 }
 
 // Where U12's column j of a leaf is staged: a tile's lanes read columns 4 q + i together, so those
@@ -156,7 +144,7 @@ __global__ void __launch_bounds__(kLppThreads, 1) lpp_panel_kernel(float* __rest
       // the warp's candidate: the largest key (redux), the lowest lane holding it (ballot);
       // every lane's reciprocal is taken while the reduction runs, the winner posts its own
       const unsigned key = active ? pivot_key(p[c]) : 0u;
-      const float myrcp = lpp_rcp(p[c]);
+      const float myrcp = __frcp_rn(active ? p[c] : 1.0f);  // 1 keeps idle rows off its long path
       const unsigned wmax = __reduce_max_sync(0xffffffffu, key);
       const int wl = __ffs(__ballot_sync(0xffffffffu, key == wmax)) - 1;
       if (lane == wl) {
