@@ -22,9 +22,10 @@ static_assert(NMAX == MAX_N, "the build's size class");
 constexpr int THREADS = NMAX;
 constexpr int WARPS = THREADS / 32;
 constexpr int KMAX = kBatchMaxK;
-// The 64-thread build takes its pivots by integer keys with the reciprocals posted, and float
-// reciprocals by approximation: those systems are bound by the latency of a column. In the 256-thread
-// build the same changes made the kernel's code longer and every phase ~8% slower, so it keeps its own.
+// The 64-thread build takes its pivots by integer keys with the reciprocals posted, and bsolve's float
+// quotients by bquotient: those systems are bound by the latency of a column. In the 256-thread build the
+// same changes made the kernel's code longer and every phase ~8% slower, so it keeps its own. (bsolve_t's
+// float quotients are bquotient's in both.)
 constexpr bool SHORT = NMAX <= 64;
 constexpr int SLOT_BYTES = SHORT ? 160 : 144;
 constexpr int UBT_BYTES = NMAX * 144;  // U12 transposed (NMAX rows of 144 bytes), or row segments
@@ -110,36 +111,35 @@ __device__ __forceinline__ T tabs(T v) {
   return v < T(0) ? -v : v;
 }
 
-// The reciprocal that rustymath's divide multiplies by; 0 where a pivot is divided by instead (a
-// subnormal one) or has a reciprocal that rounds to 0. float: the hardware's approximation and two
-// Newton steps x += x (1 - a x), the second of which rounds correctly but for a mantissa of all
-// ones (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor",
-// 1990): no branch, where the intrinsic's ~130 cycles were on the path of every column.
-__device__ __forceinline__ double brecip(double piv) { return fabs(piv) < DBL_MIN ? 0.0 : 1.0 / piv; }
-__device__ __forceinline__ float brecip(float piv) {
-  float x;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(x) : "f"(piv));
-  const float y = fmaf(x, fmaf(-piv, x, 1.0f), x);
-  const float z = fmaf(y, fmaf(-piv, y, 1.0f), y);
-  return fabsf(piv) < FLT_MIN || x == 0.0f ? 0.0f : z;
+// The reciprocal that rustymath's divide multiplies by, correctly rounded; 0 where it divides by the
+// pivot instead (a subnormal one). Those pass 1, which keeps a warp off the reciprocal's long path.
+__device__ __forceinline__ double brecip(double piv) {
+  const bool sub = fabs(piv) < DBL_MIN;
+  const double r = 1.0 / (sub ? 1.0 : piv);
+  return sub ? 0.0 : r;
 }
-// y / d from d's reciprocal rd: the product and one correction by its remainder (the same paper); the
-// product itself where that is no number (an infinite y)
-__device__ __forceinline__ float bquotient(float y, float d, float rd) {
-  const float q = y * rd, t = fmaf(fmaf(-q, d, y), rd, q);
-  return t != t ? q : t;
+__device__ __forceinline__ float brecip(float piv) {
+  const bool sub = fabsf(piv) < FLT_MIN;
+  const float r = __frcp_rn(sub ? 1.0f : piv);
+  return sub ? 0.0f : r;
 }
 // rustymath's divide: multiply by the reciprocal unless the pivot is subnormal
 __device__ __forceinline__ double bdivide(double x, double piv) {
   return fabs(piv) < DBL_MIN ? x / piv : x * (1.0 / piv);
 }
-__device__ __noinline__ float bdivide_rare(float x, float piv) { return x / piv; }
 __device__ __forceinline__ float bdivide(float x, float piv) {
-  if constexpr (SHORT) {
-    const float r = brecip(piv);
-    return r != 0.0f ? x * r : bdivide_rare(x, piv);
-  }
   return fabsf(piv) < FLT_MIN ? x / piv : x * __frcp_rn(piv);
+}
+
+// y / d, correctly rounded, from rd = 1 / d in float64: y rd lies within 2^-52 of y / d, relatively, and no
+// quotient of two floats comes within 2^-49 of a midpoint between two (of a normal quotient a midpoint m
+// has 25 bits and d 24, so the integer |y 2^s - m d| is at least 1, and it is not 0, as m d has more bits
+// than y). Subnormal quotients, where midpoints have fewer bits, are divided. The quotient is one step of
+// a serial chain over the columns: forward and adjoint of 4096 systems of n = 64, k = 2, take 1.35 ms with
+// it and 1.48 with the division in its place.
+__device__ __forceinline__ float bquotient(float y, float d, double rd) {
+  const double q = (double)y * rd;
+  return fabs(q) < (double)FLT_MIN && q != 0.0 ? y / d : (float)q;
 }
 
 // The lowest lane of the warp's largest key (hi, lo); lo counts for T = double only.
@@ -674,18 +674,19 @@ __device__ void bsolve(const T* W, int ld, int n, int k, Smem& sm, int my_pos, T
       load_row<T, NB>(W + (int64_t)(lane < nbj ? sm.piv[J + lane] : 0) * ld + J, nbj, uv);
       for_each_rhs(warp, k, [&](int c) {
         T y = lane < nbj ? (T)sm.vsm[lane][c] : T(0);
-        T rd = T(0), own = T(0);  // float: this lane's reciprocal, ahead of the chain
+        T own = T(1);  // float: this lane's divisor and its reciprocal, ahead of the chain
+        double rd = 1.0;
         if constexpr (SHORT && sizeof(T) == 4) {
 #pragma unroll
           for (int q = 0; q < NB; ++q)
-            if (q == lane) own = uv[q];
-          rd = brecip(own);
+            if (q == lane && q < nbj) own = uv[q];
+          rd = 1.0 / (double)own;
         }
 #pragma unroll
         for (int q = NB - 1; q >= 0; --q) {
           if (q < nbj) {
             if (lane == q) {
-              if constexpr (SHORT && sizeof(T) == 4) y = rd != T(0) ? bquotient(y, own, rd) : bdivide_rare(y, own);
+              if constexpr (SHORT && sizeof(T) == 4) y = bquotient(y, own, rd);
               else y = y / uv[q];
             }
             const T xq = __shfl_sync(0xffffffffu, y, q);
@@ -966,18 +967,19 @@ __device__ void bsolve_t(const T* W, int ld, int n, int k, Smem& sm, T (&v)[KMAX
         ucol[q] = (lane < nbj && q <= lane) ? W[(int64_t)sm.piv[J + q] * ld + J + lane] : T(0);
       for_each_rhs(warp, k, [&](int c) {
         T y = lane < nbj ? (T)sm.vsm[lane][c] : T(0);
-        T rd = T(0), own = T(0);  // float: this lane's reciprocal, ahead of the chain
+        T own = T(1);  // float: this lane's divisor and its reciprocal, ahead of the chain
+        double rd = 1.0;
         if constexpr (sizeof(T) == 4) {
 #pragma unroll
           for (int q = 0; q < NB; ++q)
-            if (q == lane) own = ucol[q];
-          rd = brecip(own);
+            if (q == lane && q < nbj) own = ucol[q];
+          rd = 1.0 / (double)own;
         }
 #pragma unroll
         for (int q = 0; q < NB; ++q) {
           if (q < nbj) {
             if (lane == q) {
-              if constexpr (sizeof(T) == 4) y = rd != T(0) ? bquotient(y, own, rd) : bdivide_rare(y, own);
+              if constexpr (sizeof(T) == 4) y = bquotient(y, own, rd);
               else y = y / ucol[q];
             }
             const T zq = __shfl_sync(0xffffffffu, y, q);

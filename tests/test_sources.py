@@ -7,7 +7,8 @@ import pytest
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "rustymath_b200", "csrc")
 
 
-@pytest.mark.parametrize("name", ["getrf.cu", "getrf_block.cu", "mixed.cu", "potrf.cu", "short_pivot.cuh"])
+@pytest.mark.parametrize("name", ["getrf.cu", "getrf_block.cu", "mixed.cu", "potrf.cu", "short_pivot.cuh",
+                                  "batched_kernels.cuh"])
 def test_reciprocals_are_correctly_rounded(name):
     """rustymath multiplies a pivot's column by the pivot's correctly rounded reciprocal. The kernels take it
     from CUDA's intrinsics and operators, not from the hardware's approximation."""
