@@ -14,3 +14,8 @@ def test_reciprocals_are_correctly_rounded(name):
     from CUDA's intrinsics and operators, not from the hardware's approximation."""
     (path,) = glob.glob(os.path.join(CSRC, name))
     assert "rcp.approx" not in open(path).read()
+
+
+def test_a_change_to_any_source_or_header_rebuilds_the_library():
+    from rustymath_b200 import build
+    assert set(glob.glob(os.path.join(CSRC, "*"))) <= set(build.sources() + build.headers())
