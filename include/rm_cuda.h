@@ -110,6 +110,10 @@ int rm_test_inject_failure(int kind, int after, int count);
  * own; synchronises. The device stays usable afterwards. */
 int rm_test_chain_timeout(int64_t wait_ns);
 
+/* On the calling thread, the float64 LU's leaves take clusters of at most `ctas` CTAs (a power of two up
+ * to 16; 0: as many as the device places), as on a device that places no larger ones. */
+int rm_test_limit_leaf_ctas(int ctas);
+
 /* C = alpha*op(A)*op(B) + beta*C, row-major, op(X) = X or X^T (trans* = RM_TRANS).
  * op(A) is m x k, op(B) is k x n, C is m x n. Mirrors Accelerated::xgemm
  * (core/src/linalg/accelerate.rs:211) with order fixed to row-major. */

@@ -44,6 +44,7 @@ SIGNATURES = {
     "rm_device_count": (ctypes.c_int, [ctypes.POINTER(ctypes.c_int)]),
     "rm_take_status": (ctypes.c_int, [_p]),
     "rm_test_inject_failure": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int]),
+    "rm_test_limit_leaf_ctas": (ctypes.c_int, [ctypes.c_int]),
     "rm_test_chain_timeout": (ctypes.c_int, [_i64]),
     "rm_dgemm": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, _i64, _i64, _i64, _f64, _p, _i64, _p, _i64, _f64, _p,
                                 _i64, _p]),

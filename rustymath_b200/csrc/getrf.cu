@@ -770,6 +770,7 @@ int getrf_f64(double* w, int64_t ldw, int64_t n64, int64_t* ipiv, int64_t* perm,
   // whose CTAs do not stay on the SMs where the latest leaf ran.
   F64LookAhead la;
   const bool ahead = n >= 1024;
+  const int leaf_rows = leaf_max_rows();
   cudaStream_t stream = caller;
   if (ahead) {
     RM_CUDA_TRY(cudaMemsetAsync(&gs->marks, 0, sizeof gs->marks, caller));
@@ -785,7 +786,7 @@ int getrf_f64(double* w, int64_t ldw, int64_t n64, int64_t* ipiv, int64_t* perm,
     BlockScratch* bs = &gs->block[J0 / kOuter & 1];
     for (int j0 = J0; j0 < J1; j0 += kLeaf) {
       const int jb = std::min(kLeaf, J1 - j0);
-      if (n - j0 <= kLeafMaxRows) {
+      if (n - j0 <= leaf_rows) {
         RM_TRY(leaf_f64(w, ldw, n, j0, jb, J0, J1, bs, ahead ? &gs->marks : nullptr, status, stream));
       } else {
         RM_TRY(launch_panel<double>(w, ldw, n, j0, jb, ipiv, stream));

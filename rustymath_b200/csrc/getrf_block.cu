@@ -13,6 +13,8 @@
 // has already overwritten.
 #include <algorithm>
 #include <climits>
+#include <mutex>
+#include <vector>
 
 #include "getrf_block.cuh"
 #include "rm_cluster.cuh"
@@ -416,12 +418,61 @@ __global__ void __launch_bounds__(kLeafMaxThreads, 1)
 // ~500 cycles more than 128) costs more than a wider exchange, 256 rows each up to 16 CTAs.
 constexpr int kLeafRows = 256;
 
+static cudaLaunchConfig_t leaf_config(cudaLaunchAttribute* attr, int ctas, int threads) {
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = ctas;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = leaf_smem(threads);
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+// The largest cluster of whole leaf CTAs that this device can place; a single CTA needs none.
+static int find_leaf_cluster_limit() {
+  if (smem_attribute(leaf_kernel<true>, leaf_smem(kLeafMaxThreads)) == RM_OK &&
+      func_attribute(reinterpret_cast<const void*>(leaf_kernel<true>),
+                     cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == RM_OK)
+    for (int C = kLeafMaxCtas; C > 1; C /= 2) {
+      cudaLaunchAttribute attr;
+      const cudaLaunchConfig_t cfg = leaf_config(&attr, C, kLeafMaxThreads);
+      int clusters = 0;
+      if (cudaOccupancyMaxActiveClusters(&clusters, leaf_kernel<true>, &cfg) == cudaSuccess && clusters > 0) return C;
+      cudaGetLastError();
+    }
+  cudaGetLastError();
+  return 1;
+}
+
+static thread_local int g_leaf_ctas = kLeafMaxCtas;  // lowered by tests only
+
+// Found once per device.
+static int leaf_cluster_limit() {
+  static std::mutex mu;
+  static std::vector<int> limits;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+  std::lock_guard<std::mutex> lock(mu);
+  if ((int)limits.size() <= dev) limits.resize(dev + 1, 0);
+  if (!limits[dev]) limits[dev] = find_leaf_cluster_limit();
+  return std::min(limits[dev], g_leaf_ctas);
+}
+
+int leaf_max_rows() { return leaf_cluster_limit() * kLeafMaxThreads; }
+
 int leaf_f64(double* w, int64_t ldw, int n, int j0, int jb, int J0, int J1, BlockScratch* s, LeafMarks* marks,
              unsigned* status, cudaStream_t stream) {
   const int M = n - j0;
   int C = 1;
-  if (M > kLeafMaxThreads)
-    while (C < kLeafMaxCtas && M > C * kLeafRows) C *= 2;
+  if (M > kLeafMaxThreads) {
+    const int limit = leaf_cluster_limit();
+    while (C < limit && M > C * kLeafRows) C *= 2;
+    if (M > C * kLeafMaxThreads) return RM_BAD_ARG;
+  }
   const int T = std::max(32, ((M + C - 1) / C + 31) / 32 * 32);
   if (C == 1) {
     RM_TRY(smem_attribute(leaf_kernel<false>, leaf_smem(kLeafMaxThreads)));
@@ -430,21 +481,9 @@ int leaf_f64(double* w, int64_t ldw, int n, int j0, int jb, int J0, int J1, Bloc
     note_launch();
     return RM_OK;
   }
-  RM_TRY(smem_attribute(leaf_kernel<true>, leaf_smem(kLeafMaxThreads)));
-  RM_TRY(func_attribute(reinterpret_cast<const void*>(leaf_kernel<true>),
-                        cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = C;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3(C);
-  cfg.blockDim = dim3(T);
-  cfg.dynamicSmemBytes = leaf_smem(T);
+  cudaLaunchAttribute attr;  // the kernel's attributes are set since the limit was found
+  cudaLaunchConfig_t cfg = leaf_config(&attr, C, T);
   cfg.stream = stream;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   unsigned hold = 0u;  // a self-test's leaf, with a short limit
   if (injected_failure(RM_INJECT_LEAF_TIMEOUT)) hold = 0xffffffffu;
   else if (injected_failure(RM_INJECT_LEAF_CTA_TIMEOUT)) hold = 1u << (C - 1);
@@ -484,7 +523,7 @@ __device__ __forceinline__ void move_rows(double* w, int64_t ldw, int j0, int J0
 }
 
 // The moves of a leaf whose rows were swapped one after another (ipiv, absolute): their net
-// effect, then the same buffer and lists. One CTA; only leaves taller than kLeafMaxRows come here.
+// effect, then the same buffer and lists. One CTA; only leaves taller than leaf_max_rows() come here.
 __global__ void __launch_bounds__(256) leaf_moves_kernel(double* w, int64_t ldw, int j0, int jb, int J0, int J1,
                                                          const int64_t* __restrict__ ipiv, BlockScratch* s) {
   __shared__ int pos[2 * kLeaf], src[2 * kLeaf], cnt_s;
@@ -899,3 +938,9 @@ int block_rows_f64(double* w, int64_t ldw, int J0, int nb, bool left, int lo, in
 }
 
 }  // namespace rm
+
+extern "C" int rm_test_limit_leaf_ctas(int ctas) {
+  if (ctas < 0 || ctas > rm::kLeafMaxCtas || (ctas & (ctas - 1))) return RM_BAD_ARG;
+  rm::g_leaf_ctas = ctas ? ctas : rm::kLeafMaxCtas;
+  return RM_OK;
+}

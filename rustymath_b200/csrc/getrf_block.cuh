@@ -32,8 +32,10 @@ struct LeafMarks {
   int sm[kSmMarks];
 };
 
-// Rows that leaf_f64 takes: a thread per row, 512 threads in each of 16 CTAs.
+// Rows that leaf_f64 takes: a thread per row, 512 threads in each of 16 CTAs, or of as many as the current
+// device places in one cluster.
 constexpr int kLeafMaxRows = 8192;
+int leaf_max_rows();
 
 // Factors the leaf of columns j0 .. j0 + jb (of the block J0 .. J1) over rows j0 .. n - 1, its rows
 // left at their final positions; fills s->moves[(j0 - J0) / kLeaf] and s->rows. The block's last
