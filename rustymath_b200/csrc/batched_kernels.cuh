@@ -1194,7 +1194,7 @@ __global__ void __launch_bounds__(THREADS, RM_BT_MIN_BLOCKS) batch_adjoint_kerne
     // gb (packed like b) and ga = -gb x^T (packed like a)
     double* gb = aj.gb + bt.b_off[s];
     for (int e = threadIdx.x; e < n * k; e += THREADS) gb[e] = sm.xs[e / k][e % k];
-    if (aj.ga) {
+    if (aj.ga && n > 0) {
       const double* x = bt.x + bt.x_off[s];
       for (int e = threadIdx.x; e < n * k; e += THREADS) sm.rs[e / k][e % k] = x[e];
       __syncthreads();
