@@ -22,12 +22,13 @@ static_assert(NMAX == MAX_N, "the build's size class");
 constexpr int THREADS = NMAX;
 constexpr int WARPS = THREADS / 32;
 constexpr int KMAX = kBatchMaxK;
-// The 64-thread build takes its pivots by integer keys with the reciprocals posted, and bsolve's float
-// quotients by bquotient: those systems are bound by the latency of a column. In the 256-thread build the
-// same changes made the kernel's code longer and every phase ~8% slower, so it keeps its own. (bsolve_t's
-// float quotients are bquotient's in both.)
+// The 64-thread build's float32 factors take their reciprocals posted, and bsolve's float quotients come by
+// bquotient: those systems are bound by the latency of a column. In the 256-thread build the same changes
+// made the kernel's code longer and every phase ~8% slower, and float64 factors by integer keys were slower
+// than by their magnitudes in the 64-thread one (general matrices of n = 9 .. 60, forward: 1.02 to 1.09 of
+// the time; n = 64 the same): they keep their own. (bsolve_t's float quotients are bquotient's in both.)
 constexpr bool SHORT = NMAX <= 64;
-constexpr int SLOT_BYTES = SHORT ? 160 : 144;
+constexpr int SLOT_BYTES = 144;
 constexpr int UBT_BYTES = NMAX * 144;  // U12 transposed (NMAX rows of 144 bytes), or row segments
 
 struct Smem {
@@ -113,11 +114,6 @@ __device__ __forceinline__ T tabs(T v) {
 
 // The reciprocal that rustymath's divide multiplies by, correctly rounded; 0 where it divides by the
 // pivot instead (a subnormal one). Those pass 1, which keeps a warp off the reciprocal's long path.
-__device__ __forceinline__ double brecip(double piv) {
-  const bool sub = fabs(piv) < DBL_MIN;
-  const double r = 1.0 / (sub ? 1.0 : piv);
-  return sub ? 0.0 : r;
-}
 __device__ __forceinline__ float brecip(float piv) {
   const bool sub = fabsf(piv) < FLT_MIN;
   const float r = __frcp_rn(sub ? 1.0f : piv);
@@ -135,23 +131,17 @@ __device__ __forceinline__ float bdivide(float x, float piv) {
 // quotient of two floats comes within 2^-49 of a midpoint between two (of a normal quotient a midpoint m
 // has 25 bits and d 24, so the integer |y 2^s - m d| is at least 1, and it is not 0, as m d has more bits
 // than y). Subnormal quotients, where midpoints have fewer bits, are divided. The quotient is one step of
-// a serial chain over the columns: forward and adjoint of 4096 systems of n = 64, k = 2, take 1.35 ms with
-// it and 1.48 with the division in its place.
+// a serial chain over the columns: forward and adjoint of 4096 systems of n = 64, k = 2, took 1.48 ms with
+// the division and 1.35 with this (1.29 with the float64 factors' code below out of its way).
 __device__ __forceinline__ float bquotient(float y, float d, double rd) {
   const double q = (double)y * rd;
   return fabs(q) < (double)FLT_MIN && q != 0.0 ? y / d : (float)q;
 }
 
-// The lowest lane of the warp's largest key (hi, lo); lo counts for T = double only.
-template <typename T>
-__device__ __forceinline__ int best_lane(unsigned hi, unsigned lo) {
-  const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
-  unsigned top = __ballot_sync(0xffffffffu, hi == mhi);
-  if (sizeof(T) == 8 && (top & (top - 1u))) {
-    const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
-    top = __ballot_sync(0xffffffffu, hi == mhi && lo == mlo);
-  }
-  return __ffs(top) - 1;
+// The lowest lane of the warp's largest key
+__device__ __forceinline__ int best_lane(unsigned key) {
+  const unsigned top = __reduce_max_sync(0xffffffffu, key);
+  return __ffs(__ballot_sync(0xffffffffu, key == top)) - 1;
 }
 
 template <typename T>
@@ -368,30 +358,22 @@ __device__ void bfactor_pivoted(T* W, int ld, int n, Smem& sm, int& my_pos) {
       if (c < nbj) {
         unsigned char(*sl)[SLOT_BYTES] = sm.slot[c & 1];
         int bi, bw;
-        if constexpr (SHORT) {
+        if constexpr (SHORT && sizeof(T) == 4) {
           // the largest magnitude, the lowest row among equals; a NaN only when nothing else is left.
-          // Keys: 0 no candidate, 1 NaN, else the magnitude's (high) bits + 2 and low bits. The
-          // reciprocal a winner would give is formed beside the reduction and posted.
-          unsigned hi = 0u, lo = 0u;
-          if constexpr (sizeof(T) == 4) {
-            const float v = fabsf(p[c]);
-            if (active) hi = v != v ? 1u : __float_as_uint(v) + 2u;
-          } else {
-            const unsigned long long m = (unsigned long long)__double_as_longlong(p[c]) & 0x7fffffffffffffffull;
-            if (active) hi = m > 0x7ff0000000000000ull ? 1u : (unsigned)(m >> 32) + 2u;
-            lo = hi > 1u ? (unsigned)m : 0u;
-          }
+          // Keys: 0 no candidate, 1 NaN, else the magnitude's bits + 2. The reciprocal a winner would give is
+          // formed beside the reduction and posted.
+          const float v = fabsf(p[c]);
+          const unsigned key = !active ? 0u : v != v ? 1u : __float_as_uint(v) + 2u;
           const T rcp = brecip(p[c]);
-          if (lane == best_lane<T>(hi, lo)) {
+          if (lane == best_lane(key)) {
             T* post = reinterpret_cast<T*>(sl[warp]);
 #pragma unroll
             for (int i = 0; i < NB; ++i) post[i] = p[i];
-            *reinterpret_cast<uint4*>(sl[warp] + 128) = make_uint4(hi, lo, (unsigned)r, 0u);
-            *reinterpret_cast<T*>(sl[warp] + 144) = rcp;
+            *reinterpret_cast<uint4*>(sl[warp] + 128) = make_uint4(key, __float_as_uint(rcp), (unsigned)r, 0u);
           }
           __syncthreads();
-          const uint2 post_key = lane < WARPS ? *reinterpret_cast<const uint2*>(sl[lane] + 128) : make_uint2(0u, 0u);
-          bw = best_lane<T>(post_key.x, post_key.y);  // lanes are warps, in row order
+          const unsigned post_key = lane < WARPS ? *reinterpret_cast<const unsigned*>(sl[lane] + 128) : 0u;
+          bw = best_lane(post_key);  // lanes are warps, in row order
           bi = *reinterpret_cast<const int*>(sl[bw] + 136);
         } else {
           T key = T(-1);
@@ -457,8 +439,8 @@ __device__ void bfactor_pivoted(T* W, int ld, int n, Smem& sm, int& my_pos) {
         if (active) {
           if (piv != T(0)) {
             T l;
-            if constexpr (SHORT) {
-              const T r1 = *reinterpret_cast<const T*>(sl[bw] + 144);
+            if constexpr (SHORT && sizeof(T) == 4) {
+              const T r1 = *reinterpret_cast<const T*>(sl[bw] + 132);
               l = r1 != T(0) ? p[c] * r1 : bdivide(p[c], piv);
             } else {
               l = bdivide(p[c], piv);
