@@ -9,7 +9,8 @@
 //   for each block of kOuter columns at J0 (getrf_block.cu):
 //     for each 32-column leaf at j0 inside it:
 //       leaf_kernel       : pivot search, scale and rank-1 updates of the leaf, the rows in the
-//                           registers of up to 16 CTAs (taller than 8192 rows: panel_kernel)
+//                           shared memory of up to 16 CTAs (taller than 512 rows for each CTA of
+//                           the largest cluster: panel_kernel)
 //       leaf_tail_kernel  : the leaf's row moves on the block's other columns, U = L^-1 A for the
 //                           leaf's rows of the block's later columns, and those columns' update
 //     block_rows_kernel   : the block's row moves on every column outside it, and perm; U12 =
@@ -215,10 +216,11 @@ __global__ void __launch_bounds__(kPanelThreads)
 // column by column, right-looking, with one cluster barrier per pivot column, in place of the
 // blocked path's chain of dependent launches (leaves, swaps, inversions, block products). Each
 // item takes the fmas of rustymath's packed products in the same order (one per pivot column,
-// in column order), so the factors are the oracle's bits. Measured per solve (n = 128 / 192 /
-// 256): 0.29 / 0.41 / 0.51 ms against 0.31 / 0.47 / 0.57 ms on the blocked path; a column costs
-// ~1.1 us at C = 2 and ~2.2 us at C = 16 (the cluster barrier and the pivot row's reads from one
-// CTA's shared memory), so at n = 384..512 the blocked path is faster and keeps those sizes.
+// in column order), so the factors are the oracle's bits, which is why these sizes stay here: the
+// blocked path, whose block rows go through inverted diagonal blocks, does not give them, but has become
+// the faster one (a factorization at n = 64 / 128 / 192 / 256: 0.132 / 0.203 / 0.308 / 0.422 ms here,
+// 0.106 / 0.165 / 0.243 / 0.307 ms there). A column costs ~1.1 us at C = 2 and ~2.2 us at C = 16 (the cluster
+// barrier and the pivot row's reads from one CTA's shared memory).
 //
 // Rows do not move. Every warp of a CTA tracks the positions of the CTA's rows (lane = row), so
 // a pivot choice only exchanges two positions, as in leaf_kernel; at the end each row is
@@ -527,9 +529,10 @@ __global__ void __launch_bounds__(kSmallSolveMax, 1)
   }
 }
 
-// The plain solve takes this kernel up to n = 192: measured per solve (n = 8 / 32 / 64 / 128 / 192 / 256,
-// one right-hand side) 0.051 / 0.092 / 0.142 / 0.244 / 0.380 / 0.513 ms against 0.127 / 0.155 / 0.178 /
-// 0.271 / 0.385 / 0.490 ms with the block-chained solves.
+// The plain solve takes this kernel up to n = 192, where one right-hand side gives the oracle's bits. Whole
+// solves with it and with the block-chained solves in its place (n = 64 / 128 / 192 / 256): one right-hand
+// side 0.192 / 0.288 / 0.424 / 0.586 against 0.207 / 0.283 / 0.406 / 0.519 ms, eight 0.220 / 0.348 / 0.514 /
+// 0.697 against 0.207 / 0.283 / 0.407 / 0.522 ms.
 constexpr int kSmallSolveRoute = 192;
 bool small_solve_fits(int64_t n, int64_t k) { return n >= 1 && n <= kSmallSolveRoute && k >= 1 && k <= kSmallSolveK; }
 

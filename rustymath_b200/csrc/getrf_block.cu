@@ -1,7 +1,7 @@
 // One 128-column block of the blocked float64 LU: leaves of 32 columns, and the block's rows.
 //
 // A block is a chain of small dependent steps, so what counts is the number of launches and the
-// latency inside each. Per leaf: leaf_kernel (pivoting and factorization, the rows in registers)
+// latency inside each. Per leaf: leaf_kernel (pivoting and factorization, the rows in shared memory)
 // and leaf_tail_kernel (the row moves, U12 and the rank-32 update of the block's later columns in
 // one launch); per block: block_rows_kernel (the row moves of all four leaves on the other
 // columns and U12 = L11^-1 A12). The trailing update is dgemm's.
@@ -493,29 +493,29 @@ int leaf_f64(double* w, int64_t ldw, int n, int j0, int jb, int J0, int J1, Bloc
   return RM_OK;
 }
 
-// The block's other columns of the moved rows first, first + step, ... below cnt into s->rows (or,
-// with SCATTER, the columns left of the leaf from there to their new positions), 16 bytes per
-// thread and four in flight. pos: the rows relative to base; at: the first row's slot.
+// The block's other columns of the cnt moved rows into s->rows (or, with SCATTER, the columns left of the
+// leaf from there to their new positions), 16 bytes per thread and four in flight. pos: the rows relative
+// to j0; at: the first row's slot.
 template <bool SCATTER>
 __device__ __forceinline__ void move_rows(double* w, int64_t ldw, int j0, int J0, BlockScratch* s, const int* pos,
-                                          int base, int first, int step, int cnt, int at) {
+                                          int cnt, int at) {
   constexpr int kPer = kOuter / 2;  // 16-byte pieces of a row
-  const int total = cnt > first ? ((cnt - first + step - 1) / step) * kPer : 0;
+  const int total = cnt * kPer;
   const int lc = (j0 - J0) / 2;  // the leaf's first piece
   for (int e0 = threadIdx.x; e0 < total; e0 += 4 * (int)blockDim.x) {
     double2 v[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int e = e0 + u * (int)blockDim.x, i = first + e / kPer * step, q = e % kPer;
+      const int e = e0 + u * (int)blockDim.x, i = e / kPer, q = e % kPer;
       if (e < total && (q < lc || (!SCATTER && q >= lc + kLeaf / 2)))
         v[u] = SCATTER ? *reinterpret_cast<const double2*>(&s->rows[at + i][2 * q])
-                       : *reinterpret_cast<const double2*>(w + (int64_t)(base + pos[i]) * ldw + J0 + 2 * q);
+                       : *reinterpret_cast<const double2*>(w + (int64_t)(j0 + pos[i]) * ldw + J0 + 2 * q);
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int e = e0 + u * (int)blockDim.x, i = first + e / kPer * step, q = e % kPer;
+      const int e = e0 + u * (int)blockDim.x, i = e / kPer, q = e % kPer;
       if (e < total && (q < lc || (!SCATTER && q >= lc + kLeaf / 2))) {
-        if constexpr (SCATTER) *reinterpret_cast<double2*>(w + (int64_t)(base + pos[i]) * ldw + J0 + 2 * q) = v[u];
+        if constexpr (SCATTER) *reinterpret_cast<double2*>(w + (int64_t)(j0 + pos[i]) * ldw + J0 + 2 * q) = v[u];
         else *reinterpret_cast<double2*>(&s->rows[at + i][2 * q]) = v[u];
       }
     }
@@ -550,16 +550,16 @@ __global__ void __launch_bounds__(256) leaf_moves_kernel(double* w, int64_t ldw,
   }
   __syncthreads();
   const int disp = cnt_s - jb;
-  move_rows<false>(w, ldw, j0, J0, s, src, j0, 0, 1, jb, 0);
-  move_rows<false>(w, ldw, j0, J0, s, src + jb, j0, 0, 1, disp, kLeaf);
+  move_rows<false>(w, ldw, j0, J0, s, src, jb, 0);
+  move_rows<false>(w, ldw, j0, J0, s, src + jb, disp, kLeaf);
   LeafMoves& mv = s->moves[(j0 - J0) / kLeaf];
   if (t == 0) mv.j0 = j0, mv.jb = jb, mv.disp = disp;
   if (t < jb) mv.piv_src[t] = j0 + src[t];
   if (t < disp) mv.disp_src[t] = j0 + src[jb + t], mv.disp_dst[t] = j0 + pos[jb + t];
   __syncthreads();
   if (j0 + jb == J1 && j0 > J0) {
-    move_rows<true>(w, ldw, j0, J0, s, pos, j0, 0, 1, jb, 0);
-    move_rows<true>(w, ldw, j0, J0, s, pos + jb, j0, 0, 1, disp, kLeaf);
+    move_rows<true>(w, ldw, j0, J0, s, pos, jb, 0);
+    move_rows<true>(w, ldw, j0, J0, s, pos + jb, disp, kLeaf);
   }
 }
 

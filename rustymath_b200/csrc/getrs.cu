@@ -22,9 +22,9 @@ constexpr int kPreKC = 8;           // columns per chain of the scaled float32 s
 size_t diag_blocks_f64_bytes(int64_t n) { return diag_blocks_bytes_max(n); }
 
 // out (TB x TB, row-major, ld ldo) = dinv block dv (TB x TB row-major) times block (b, pb) of
-// the n x n matrix T (item (i, j) at w[i*ldw + j], or at w[j*ldw + i] when COLMAJOR; past n,
-// zero). 256 threads, each a (TB/16)^2 piece; smem holds both operands.
-template <typename T, bool COLMAJOR, int TB>
+// the row-major n x n matrix w (past n, zero). 256 threads, each a (TB/16)^2 piece; smem holds both
+// operands.
+template <typename T, int TB>
 __device__ __forceinline__ void block_product(const T* __restrict__ w, int64_t ldw, int64_t n, int b, int pb,
                                               const T* __restrict__ dv, T* __restrict__ out, int64_t ldo) {
   constexpr int R = TB / 16;
@@ -35,10 +35,8 @@ __device__ __forceinline__ void block_product(const T* __restrict__ w, int64_t l
   for (int e = threadIdx.x; e < TB * TB; e += 256) {
     const int i = e / TB, j = e % TB;
     di[i][j] = dv[e];
-    // COLMAJOR storage read down its columns (coalesced)
-    const int ri = COLMAJOR ? j : i, cj = COLMAJOR ? i : j;
-    const int64_t gi = r0 + ri, gj = c0 + cj;
-    ob[ri][cj] = (gi < n && gj < n) ? (COLMAJOR ? w[gj * ldw + gi] : w[gi * ldw + gj]) : T(0);
+    const int64_t gi = r0 + i, gj = c0 + j;
+    ob[i][j] = (gi < n && gj < n) ? w[gi * ldw + gj] : T(0);
   }
   __syncthreads();
   const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
@@ -68,15 +66,15 @@ __device__ __forceinline__ void block_product(const T* __restrict__ w, int64_t l
 // block b to the block the forward (backward) solve finishes just before it, so that block
 // b's last step is x_b = z_b - coupling x_prev with z_b formed while it waits. A CTA per
 // (block, triangle).
-template <typename T, bool COLMAJOR, int TB>
+template <typename T, int TB>
 __global__ void __launch_bounds__(256) coupling_kernel(const T* __restrict__ w, int64_t ldw, int64_t n,
                                                        T* __restrict__ dinv) {
   const int b = blockIdx.x, which = blockIdx.y;  // 0: lower (block b-1), 1: upper (block b+1)
   const int nblk = (int)((n + TB - 1) / TB);
   const int pb = which == 0 ? b - 1 : b + 1;
   if (pb < 0 || pb >= nblk) return;
-  block_product<T, COLMAJOR, TB>(w, ldw, n, b, pb, dinv + ((int64_t)b * kDiagMats + which) * TB * TB,
-                                 dinv + ((int64_t)b * kDiagMats + 2 + which) * TB * TB, TB);
+  block_product<T, TB>(w, ldw, n, b, pb, dinv + ((int64_t)b * kDiagMats + which) * TB * TB,
+                       dinv + ((int64_t)b * kDiagMats + 2 + which) * TB * TB, TB);
 }
 
 
@@ -835,8 +833,8 @@ int couplings_f32(const float* w, int64_t ldw, int64_t n, float* dinv, cudaStrea
   const int nblk = (int)((n + kTB32 - 1) / kTB32);
   if (nblk < 2) return RM_OK;
   const size_t smem = (size_t)kTB32 * (kTB32 + 1) * sizeof(float);
-  RM_TRY(smem_attribute(coupling_kernel<float, false, kTB32>, 2 * smem));
-  coupling_kernel<float, false, kTB32><<<dim3((unsigned)nblk, 2), 256, 2 * smem, stream>>>(w, ldw, n, dinv);
+  RM_TRY(smem_attribute(coupling_kernel<float, kTB32>, 2 * smem));
+  coupling_kernel<float, kTB32><<<dim3((unsigned)nblk, 2), 256, 2 * smem, stream>>>(w, ldw, n, dinv);
   RM_LAUNCHED();
   return RM_OK;
 }

@@ -8,13 +8,14 @@
 //   C_ij ~= 2^(ea[i]+eb[j]) sum_{d<s} 2^-7(d+2) sum_{p+q=d} (A_p B_q)_ij,
 // dropping the products of order p + q >= s (below 2^-7s relative, as the truncation). The
 // inner sums are int8 x int8 products accumulated in int32 by tcgen05.mma kind::i8 - exact
-// while (d+1) k 127^2 < 2^31, so k is cut into chunks that keep it so - and each order d is
-// one persistent launch whose epilogue adds 2^(ea+eb-7(d+2)) acc to C in float64, the
-// smallest orders first. With s = 8 the truncation (2^-56 relative to 2^(ea+eb)) is below
+// while (d+1) k 127^2 < 2^31, so k is cut into chunks that keep it so - and two orders
+// d, d - 1 are one persistent launch whose epilogue adds 2^(ea+eb-7(d+2)) acc of each to C in float64,
+// the smallest first. With s = 8 the truncation (2^-56 relative to 2^(ea+eb)) is below
 // float64 rounding.
 //
-// The slices live in one scratch buffer: A's as s stacked (mp x kp) int8 planes (rows and
-// k padded with zeros to whole tiles), B's transposed (K-major) as s stacked (np x kp) planes.
+// The slices live in one scratch buffer: A's as s stacked (mp x kp) int8 planes, B's
+// transposed (K-major) as s stacked (np x kp) planes, all of whole tiles. A's columns past k are zeros; the rest
+// of the padding is not written, as it meets only those or what is not stored.
 // rustymath's matmul is float64 throughout (core/src/linalg.rs:1119-1132); this is the
 // split-precision product measured against the native float64 GEMM (rm_dgemm).
 #include <algorithm>

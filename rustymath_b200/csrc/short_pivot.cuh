@@ -1,4 +1,4 @@
-// The pivot choice of the float64 panels: a candidate's key is its magnitude's bits plus an offset
+// The pivot choice of the one-launch cluster LU: a candidate's key is its magnitude's bits plus an offset
 // (so that keys order as magnitudes do and 0 means "no candidate"); of equal keys the lowest
 // position wins, as rustymath's `largest` (factor.rs:476).
 #pragma once
@@ -20,7 +20,7 @@ __device__ __forceinline__ int short_reduce(unsigned long long key, unsigned pos
   return __ffs(__ballot_sync(0xffffffffu, tie && pos == pmin)) - 1;
 }
 
-// 1 / pivot as the cluster panel forms it (0 for a subnormal pivot, which is divided by)
+// 1 / pivot, correctly rounded (0 for a subnormal pivot, which is divided by)
 __device__ __forceinline__ double short_rcp(double pv) {
   return fabs(pv) < 2.2250738585072014e-308 ? 0.0 : __drcp_rn(pv);
 }
